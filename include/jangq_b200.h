@@ -244,9 +244,9 @@ int jq_moe_gemm(const void* x_sorted, int act_dtype, int64_t max_rows, int64_t l
                 const void* const* scales_tab, const void* const* biases_tab, const int32_t* bits_tab,
                 int sidecar_dtype, int64_t N, int64_t K, int bits, int group_size, void* y_sorted,
                 int64_t ldy, jq_stream_t stream);
-/* jq_moe_gemm over a tile list of tile_m rows per entry (the tile_m given to jq_moe_sort): 128, or 256 -- one CTA
- * then carries two 128-row accumulators and every dequantized weight tile feeds both, which pays once experts hold
- * more than 128 rows (bf16 activations and N >= 256 only; JQ_EUNSUPPORTED otherwise). */
+/* jq_moe_gemm over a tile list of tile_m rows per entry (the tile_m given to jq_moe_sort): 128, 192 -- the largest tile
+ * that one pass over an expert's weights serves -- or 256 (two tiles of 128; bf16 activations and N >= 256 only,
+ * JQ_EUNSUPPORTED otherwise). */
 int jq_moe_gemm_tiled(const void* x_sorted, int act_dtype, int64_t max_rows, int64_t ldx,
                       const int32_t* expert_offsets, const int32_t* tile_expert, const int32_t* tile_row0,
                       const int32_t* num_tiles, int64_t max_tiles, int tile_m, const uint32_t* const* codes_tab,
@@ -254,6 +254,19 @@ int jq_moe_gemm_tiled(const void* x_sorted, int act_dtype, int64_t max_rows, int
                       int sidecar_dtype, int64_t N, int64_t K, int bits, int group_size, void* y_sorted,
                       int64_t ldy, jq_stream_t stream);
 
+/* Gate and up projections of the routed experts with the SwiGLU between them, in one launch over expert-sorted rows:
+ *     h[p, n] = silu(min(g, limit)) * clip(u, -limit, limit) * (weights ? weights[order[p]] : 1),
+ *     g = deq(gate[e]) . x[p],  u = deq(up[e]) . x[p]          (jang_tools/dsv41/model.py:1216-1226)
+ * Both sums stay in float32 until h is rounded (jq_moe_gemm + jq_moe_swiglu round them to the activation type first).
+ * limit <= 0 disables the clamp.  Both banks share N, K, bits and group_size; other arguments as jq_moe_gemm_tiled. */
+int jq_moe_gate_up_swiglu(const void* x_sorted, int act_dtype, int64_t max_rows, int64_t ldx,
+                          const int32_t* expert_offsets, const int32_t* tile_expert, const int32_t* tile_row0,
+                          const int32_t* num_tiles, int64_t max_tiles, int tile_m,
+                          const uint32_t* const* gate_codes, const void* const* gate_scales,
+                          const void* const* gate_biases, const uint32_t* const* up_codes,
+                          const void* const* up_scales, const void* const* up_biases, int sidecar_dtype, int64_t N,
+                          int64_t K, int bits, int group_size, const float* weights, const int32_t* order,
+                          float limit, void* h, int64_t ldh, jq_stream_t stream);
 
 /* jq_moe_gemm without any workspace.  No counterpart in the reference (MLX allocates inside
  * gather_qmm); it exists for callers that must not allocate device memory on the request path:

@@ -24,6 +24,7 @@ JQ_GATHER_FEW_LOCAL = 2
 QGEMV_MAX_M = 16
 QGEMV_MAX_BATCH = 8
 MOE_TILE_M = 128
+MOE_GEMM_TILE_M = 192   # rows per tile of the grouped GEMMs (jq_moe_gemm_tiled, jq_moe_gate_up_swiglu)
 
 _DTYPE_ID = {torch.float32: JQ_F32, torch.float16: JQ_F16, torch.bfloat16: JQ_BF16}
 
@@ -80,6 +81,8 @@ SIGNATURES = {
                               _p, _i64, _p]),
     "jq_moe_gemm_tiled": (C.c_int, [_p, _i32, _i64, _i64, _p, _p, _p, _p, _i64, _i32, _p, _p, _p, _p, _i32, _i64, _i64, _i32,
                                     _i32, _p, _i64, _p]),
+    "jq_moe_gate_up_swiglu": (C.c_int, [_p, _i32, _i64, _i64, _p, _p, _p, _p, _i64, _i32, _p, _p, _p, _p, _p, _p, _i32, _i64,
+                                        _i64, _i32, _i32, _p, _p, C.c_float, _p, _i64, _p]),
     "jq_moe_gemm_static": (C.c_int, [_p, _i32, _i64, _i64, _p, _i32, _p, _p, _p, _p, _i32, _i64, _i64, _i32, _i32, _p,
                                      _i64, _p]),
     "jq_moe_swiglu": (C.c_int, [_p, _p, _i64, _p, _p, _p, _p, _i64, _i64, _i64, C.c_float, _i32, _p]),

@@ -1,31 +1,39 @@
 // K3: prefill-shaped quantized GEMM  Y[M,N] = X[M,K] . deq(W)[N,K]^T  on the 5th-generation
-// tensor cores (tcgen05.mma, accumulator in tensor memory).
+// tensor cores (tcgen05.mma), weights as the A operand in tensor memory.
 //
-// Bound: dense bf16/f16 tensor throughput for large M; 2*M*N*K flops per launch.
+// Bound: dense bf16/f16 tensor throughput for large M (2*M*N*K flops); for few rows the rate at which the
+// packed codes are expanded.
 //
-// One CTA computes a 128 (M) x BN (N) tile of Y.  Warp roles:
-//   warp 0        TMA producer: one elected lane copies the 128 x 64 activation tile of every
-//                 k-block into a 128-byte-swizzled shared-memory stage (cp.async.bulk.tensor);
-//   warp 1        allocates BN columns of tensor memory; one elected lane issues the MMAs
-//                 (4 x tcgen05.mma M=128, N=BN, K=16 per k-block) and commits their completion to
-//                 the mbarriers that free the stages;
-//   warps 2..     dequantizers, one weight row per thread: packed codes -> registers -> exact
-//                 q (16-bit float) -> fma(q, scale, bias) rounded once to the activation type ->
-//                 the K-major, 128-byte-swizzled B tile in shared memory (the layout TMA would
-//                 have produced), then fence.proxy.async + mbarrier arrive; afterwards the same
-//                 warps run the epilogue: tcgen05.ld the accumulator, convert, store Y.
+// The dequantized weight is the A operand: a weight row is a TMEM lane, so a dequantizer thread expands the 64 codes of
+// its row and k-block in registers and stores them with one tcgen05.st -- no shared-memory tile, no proxy fence, and the
+// MMAs read only the activations from shared memory.  The activations are the B operand, so the MMA's N is the number
+// of activation rows rounded up to 16: a short batch or a short expert costs no padded work, and one 128-row weight
+// tile feeds up to 256 of them.  Warp roles:
+//   warp 0        TMA producer: copies the activation tile of every k-block into a 128-byte-swizzled stage;
+//   warp 1        allocates the tensor memory; one elected lane issues the MMAs (M = 128, N <= 256, K = 16) and commits
+//                 their completion to the mbarriers that free the stages and the A slots;
+//   warps 2, 3    code loaders: coalesced 16-byte cp.async of the packed rows and small copies of their scales and
+//                 biases, six stages deep, completion counted on mbarriers (no barrier between warps);
+//   dequantizers  four groups of four warps, one weight row per thread: group g takes k-blocks g, g + 4, ... and owns
+//                 A slot g.
+// Two forms: one tile per CTA with an optional split of K over a cluster (dense products), and a persistent one that
+// walks the tiles of the routed experts.
 // Every mbarrier wait is bounded; a wait that runs out sets the library's status word and the
 // CTA leaves through the common exit (tensor memory is always released).
 //
-// Numerics: the B operand is the dequantized weight rounded to the activation type (what
-// MLX's qmm feeds its matrix units), products are accumulated in f32.
+// Measured (B200, N x K): 4096 rows, 14336x4096 4-bit 492 -> 364 us (978 -> 1322 TFLOP/s); 512 rows, 11008x4096 2-bit
+// 68 -> 50 us; 333 rows, 4096x4096 8-bit f16 55 -> 20 us; 61 rows, 4096x4096 6-bit 34 -> 12 us (before: the dequantized
+// tile as the B operand in shared memory, one thread per weight row, one group of dequantizer warps).
+//
+// Numerics: the A operand is the dequantized weight rounded once to the activation type (what
+// MLX's qmm feeds its matrix units), products are accumulated in f32 in ascending k order.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
-#include "jq_mma.cuh"
-#include "jq_tc.cuh"
+#include "jq_ts.cuh"
 
 namespace jq {
 
@@ -33,7 +41,6 @@ namespace jq {
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;
 constexpr int GEMM_SMEM = 227 * 1024;   // dynamic shared memory of one CTA
-constexpr int GEMM_SB = 2;     // dequantized-weight stages
 
 struct GemmArgs {
     const uint32_t* codes;
@@ -42,7 +49,11 @@ struct GemmArgs {
     void* y;
     int64_t M, N, K, ldy;
     int gs, G;
-    int y_vec_ok;    // rows of y are 16-byte aligned
+    int tn;          // activation rows per tile (multiple of 16, <= TNMAX)
+    int sub;         // grouped mode: tiles of tn rows per entry of the tile list
+    int box_rows;    // activation rows per TMA box: tn, or 32 when the rows of a tile vary (grouped mode)
+    int y_pair_ok;   // rows of y are 4-byte aligned
+    int y_vec_ok;    // rows of y are 8-byte aligned
     int* status;     // device status word, set to 1 when a bounded wait ran out
     // grouped mode (routed experts): blockIdx.y indexes a tile list built by jq_moe_sort; rows are the
     // expert-sorted (token, slot) pairs, weights come from per-expert pointer tables
@@ -54,199 +65,192 @@ struct GemmArgs {
     const void* const* scales_tab;
     const void* const* biases_tab;
     const int32_t* bits_tab;       // optional per-expert bit width: tiles of other widths exit
+    // gate/up mode (GU): the tables above are the gate's, these the up projection's; y = h of
+    // h[p, n] = silu(min(g, lim)) * clip(u, -lim, lim) * wts[order[p]]  (dsv41/model.py:1216-1226)
+    const uint32_t* const* codes_tab2;
+    const void* const* scales_tab2;
+    const void* const* biases_tab2;
+    const float* wts;
+    const int32_t* order;
+    float lim;
 };
 
-template <typename AT> __host__ __device__ constexpr uint32_t umma_fmt();
-template <> __host__ __device__ constexpr uint32_t umma_fmt<__nv_bfloat16>() { return 1u; }
-template <> __host__ __device__ constexpr uint32_t umma_fmt<__half>() { return 0u; }
-
-template <typename AT, int BN>
-__host__ __device__ constexpr uint32_t umma_idesc() {
-    return (1u << 4) /* D = f32 */ | (umma_fmt<AT>() << 7) | (umma_fmt<AT>() << 10) | ((uint32_t)(BN >> 3) << 17) |
-           ((uint32_t)(GEMM_BM >> 4) << 24);             // A and B both K-major, no negate, dense
-}
-
-// ---- packed 16-bit float helpers --------------------------------------------------------------------
-template <typename AT> struct P2;
-template <> struct P2<__nv_bfloat16> {
-    __device__ static __forceinline__ uint32_t sub(uint32_t a, uint32_t b) {
-        uint32_t r;
-        asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-        return r;
+// Scales and biases of one weight row: from the staged chunk (jq_ts.cuh), or, where rows are not staged, loaded one
+// k-block of this thread ahead (both scales of a k-block with groups of 32).
+struct Sidecars {
+    const uint16_t *srow, *brow;
+    int gs, mode;
+    uint32_t ns, nb;              // not staged: the next k-block's, one per half
+    __device__ __forceinline__ void row(const void* scales, const void* biases, int64_t n, int64_t G) {
+        srow = reinterpret_cast<const uint16_t*>(scales) + n * G;
+        brow = reinterpret_cast<const uint16_t*>(biases) + n * G;
     }
-    __device__ static __forceinline__ uint32_t fma(uint32_t a, uint32_t b, uint32_t c) {
-        uint32_t r;
-        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-        return r;
-    }
-};
-template <> struct P2<__half> {
-    __device__ static __forceinline__ uint32_t sub(uint32_t a, uint32_t b) {
-        uint32_t r;
-        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-        return r;
-    }
-    __device__ static __forceinline__ uint32_t fma(uint32_t a, uint32_t b, uint32_t c) {
-        uint32_t r;
-        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-        return r;
+    __device__ __forceinline__ void fetch(int kb) {
+        const int g = gs == 32 ? 2 * kb : gs == 64 ? kb : kb >> 1;
+        ns = __ldg(srow + g);
+        nb = __ldg(brow + g);
+        if (gs == 32) {
+            ns |= (uint32_t)__ldg(srow + g + 1) << 16;
+            nb |= (uint32_t)__ldg(brow + g + 1) << 16;
+        }
     }
 };
 
-// 32 bits of a row's code stream starting at bit A (negative A: zero-filled below bit 0)
-template <int NWORDS, int A>
-__device__ __forceinline__ uint32_t stream_at(const uint32_t (&u)[NWORDS]) {
-    if constexpr (A < 0) return u[0] << (-A);
-    else if constexpr (A % 32 == 0) return u[A / 32];
-    else if constexpr (A / 32 + 1 < NWORDS) return __funnelshift_r(u[A / 32], u[A / 32 + 1], A % 32);
-    else return u[A / 32] >> (A % 32);
-}
-
-// Weights J and J+1 of a 64-code unit: rn(q*s + bias) in the activation type, packed.
-// sp2 = (s', s') with s' = s * 2^-TGT, b2 = (bias, bias); s/bias are the same values in f32.
-template <typename AT, int BITS, int J>
-__device__ __forceinline__ uint32_t dequant_pair(const uint32_t (&u)[2 * BITS], uint32_t sp2, uint32_t b2, float s,
-                                                 float bias) {
-    if constexpr (BITS <= Act<AT>::MANT) {
-        constexpr int TGT = Act<AT>::MANT - BITS;
-        constexpr uint32_t MASK = (((1u << BITS) - 1u) << TGT) * 0x00010001u;
-        const uint32_t lo = stream_at<2 * BITS, J * BITS - TGT>(u);
-        const uint32_t hi = stream_at<2 * BITS, (J + 1) * BITS - TGT>(u);
-        const uint32_t v = and_or(prmt(lo, hi, 0x5410), MASK, Act<AT>::MAGIC);   // 2^MANT + q*2^TGT, twice
-        const uint32_t q2 = P2<AT>::sub(v, Act<AT>::MAGIC);                       // q * 2^TGT, exact
-        return P2<AT>::fma(q2, sp2, b2);                                          // one rounding
-    } else {
-        // codes wider than the mantissa (8-bit with bf16): exact q in f32 through the 2^23 trick
-        static_assert(BITS == 8, "only 8-bit codes take the f32 route");
-        const uint32_t word = u[J / 4];
-        const float q0 = __uint_as_float(prmt(word, 0x4B000000u, 0x7540u | (uint32_t)(J % 4))) - 8388608.0f;
-        const float q1 = __uint_as_float(prmt(word, 0x4B000000u, 0x7540u | (uint32_t)(J % 4 + 1))) - 8388608.0f;
-        return Act<AT>::pack_hi(fmaf(q0, s, bias), fmaf(q1, s, bias));
-    }
-}
-
-// codes 8C .. 8C+7 -> one 16-byte chunk of the B tile
-template <typename AT, int BITS, int C>
-__device__ __forceinline__ uint4 dequant_chunk(const uint32_t (&u)[2 * BITS], uint32_t sp2, uint32_t b2, float s,
-                                               float bias) {
-    return make_uint4(dequant_pair<AT, BITS, 8 * C + 0>(u, sp2, b2, s, bias),
-                      dequant_pair<AT, BITS, 8 * C + 2>(u, sp2, b2, s, bias),
-                      dequant_pair<AT, BITS, 8 * C + 4>(u, sp2, b2, s, bias),
-                      dequant_pair<AT, BITS, 8 * C + 6>(u, sp2, b2, s, bias));
-}
-
-// Code staging of one CTA: k-blocks per stage, bytes per row and stage, row pitch.  With two row tiles per CTA
-// the activation stages take twice the room, so the code stages shrink: rows of 128 bytes lose their padding
-// (their 16-byte chunks are XOR-swizzled by the row instead) and the wide odd widths stage fewer k-blocks.
-// Rows of 128 bytes are not padded there: their 16-byte chunks are XOR-swizzled by the row instead, so that the
-// eight rows a quarter-warp reads together fall into eight different 16-byte bank groups.
-// Measured on 4096x14336x4096 (B200, 4-bit): three activation stages with these code stages run at 961 TFLOP/s;
-// halving the code stages to make room for a fourth activation stage runs at 830 -- the pace is set by the
-// dequantizer warps and their per-stage synchronisation, not by the depth of the TMA pipeline; two threads per
-// weight row (twice the dequantizer warps) run at 840.
-template <int BITS, int BN, int MT> struct CodeStage {
-    static constexpr int CKB = MT == 1 ? (BITS == 2 ? 8 : (BITS == 8 ? 2 : 4))
-                                       : (BITS == 2 ? 8 : (BITS == 3 || BITS == 4) ? 4 : 2);
-    static constexpr int RB = CKB * 8 * BITS;
-    static constexpr bool SWZ = MT == 2 && RB == 128;
-    static constexpr int RBP = SWZ ? RB : RB + 16;
-    static constexpr int SA = 3;                                    // activation stages
-    static constexpr size_t SMEM = 1024 + 256 + (size_t)SA * MT * GEMM_BM * GEMM_BK * 2 + GEMM_SB * BN * GEMM_BK * 2 +
-                                   2 * BN * RBP;
-};
-
-__device__ __forceinline__ void gemm_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_cluster_f32x4(const float* own, uint32_t rank) {
-    uint32_t remote;
-    float4 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(own)), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
-    return v;
-}
-constexpr int KS_PITCH = 256 + 4;     // floats per staged accumulator row: 16 bytes of skew keep 16-byte accesses apart
-
-// MT: 128-row tiles of the activations per CTA (1 or 2).  With 2 every dequantized weight tile feeds two
-// accumulators (2 x BN columns of tensor memory), which halves the dequantizer work per flop: the kernel is
-// bound by the dequantizer warps, not by the tensor pipe, with one.
-// KS: CTAs of a cluster (along blockIdx.z) that split K, for grids that would leave most SMs idle: every CTA
-// accumulates its share of the k-blocks in its own tensor memory; the others stage their accumulators as float32
-// in their (by then idle) shared memory, and CTA 0 of the cluster adds them through distributed shared memory
-// in rank order and stores the tile.  Both cluster barriers are reached by every thread on every path.
-template <typename AT, int BITS, int BN, int DPR, int MT, int KS = 1>
-__global__ void __launch_bounds__(64 + BN * DPR)
-qgemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
+// The 64 codes of row r and k-block kb (block kbi of the staged row at crow) -> 32 registers of dequantized weights.
+// side: this row's staged chunk; kb_next: the thread's next k-block, or -1.
+template <typename AT, int BITS>
+__device__ __forceinline__ void expand_block(const uint8_t* crow, int r, int kbi, int kb, int kb_next, const uint16_t* side,
+                                             Sidecars& sc, uint32_t (&out)[32]) {
     using A = Act<AT>;
-    using CS = CodeStage<BITS, BN, MT>;
-    constexpr int GEMM_SA = CS::SA;
-    constexpr int NDW = BN / 32 * DPR;                  // dequantizer warps (DPR threads share a weight row)
-    constexpr int NDT = NDW * 32;
-    constexpr int A_TILE = GEMM_BM * GEMM_BK * 2;       // 16 KB
-    constexpr int A_STAGE = MT * A_TILE;
-    constexpr int B_STAGE = BN * GEMM_BK * 2;
-    constexpr int UW = 2 * BITS;                        // words of one row's 64 codes
-    // packed codes are staged through shared memory, CKB k-blocks at a time, so that the global
-    // reads are coalesced 16-byte chunks (8+ lanes per row) instead of one sector per thread
-    constexpr int CKB = CS::CKB;
-    constexpr int RB = CS::RB;                          // bytes per row and code stage (80..192)
-    constexpr int RBP = CS::RBP;                        // padded pitch (or swizzled chunks): conflict-free row reads
-    constexpr bool SWZ = CS::SWZ;
-    constexpr int CPR = RB / 16;                        // 16-byte chunks per row
-    constexpr int C_STAGE = BN * RBP;
-    static_assert(MT * BN <= 512, "tensor memory holds 512 columns");
-    // swizzle of a staged 128-byte code row (8 chunks): by the row
-    auto swz_of = [](int row) { return row & 7; };
+    constexpr int UW = 2 * BITS, CPR = CodeStage<BITS>::RB / 16;
+    uint32_t cur[UW];
+    if constexpr (UW % 4 == 0) {
+        const uint4* cp = reinterpret_cast<const uint4*>(crow);
+#pragma unroll
+        for (int w = 0; w < UW / 4; ++w) {
+            const uint4 v = cp[code_chunk<CPR>(kbi * (UW / 4) + w, r)];
+            cur[4 * w] = v.x; cur[4 * w + 1] = v.y; cur[4 * w + 2] = v.z; cur[4 * w + 3] = v.w;
+        }
+    } else {
+        const uint2* cp = reinterpret_cast<const uint2*>(crow + kbi * 8 * BITS);
+#pragma unroll
+        for (int w = 0; w < UW / 2; ++w) {
+            const uint2 v = cp[w];
+            cur[2 * w] = v.x; cur[2 * w + 1] = v.y;
+        }
+    }
+    uint16_t s0h, b0h, s1h, b1h;
+    if (sc.mode != 0) {
+        const int i = sc.mode == 3 ? (kb & 3) >> 1 : kb & 3;
+        s0h = s1h = side[i];
+        b0h = b1h = side[128 * 4 + i];
+    } else {
+        s0h = (uint16_t)sc.ns; b0h = (uint16_t)sc.nb;
+        s1h = sc.gs == 32 ? (uint16_t)(sc.ns >> 16) : s0h;
+        b1h = sc.gs == 32 ? (uint16_t)(sc.nb >> 16) : b0h;
+        if (kb_next >= 0) sc.fetch(kb_next);
+    }
+    const float s0 = A::to_f32(s0h), s1 = A::to_f32(s1h);
+    const uint32_t bb0 = (uint32_t)b0h * 0x00010001u, bb1 = (uint32_t)b1h * 0x00010001u;
+    // scales too large for the fast form (or not finite) send the warp's k-block through the general one
+    const bool fast = sc.gs >= 64 && __all_sync(0xFFFFFFFFu, fabsf(s0) < fast_limit<AT, BITS>());
+    if (fast) {
+        dequant_fast<AT, BITS, 2>(cur, s0, bb0, out);
+    } else {
+        const uint32_t sp0 = A::pack_hi(s0, s0), sp1 = A::pack_hi(s1, s1);
+        dequant_general<AT, BITS, 0, 0>(cur, sp0, bb0, s0, A::to_f32(b0h), out);
+        dequant_general<AT, BITS, 16, 0>(cur, sp1, bb1, s1, A::to_f32(b1h), out);
+    }
+}
+
+// 32 accumulator columns (activation rows row0 .. row0 + 31 of y, `rows` of them valid) of one weight row per lane
+template <typename AT>
+__device__ __forceinline__ void store_columns(const GemmArgs& a, const uint32_t (&v)[32], int64_t row0, int rows, int64_t nn,
+                                              bool whole, int lane) {
+    using A = Act<AT>;
+    uint16_t* yb = reinterpret_cast<uint16_t*>(a.y) + row0 * a.ldy;
+    if (a.y_pair_ok && whole) {
+        // neighbouring lanes swap halves: an even lane stores rows (n, n+1) of the even columns, an
+        // odd lane (n-1, n) of the odd ones, 4 bytes each
+        const bool odd = lane & 1;
+        uint16_t* yl = yb + (odd ? a.ldy : 0) + (nn & ~1ll);
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+            const float keep = __uint_as_float(odd ? v[j + 1] : v[j]);
+            const float got = __uint_as_float(__shfl_xor_sync(0xFFFFFFFFu, odd ? v[j] : v[j + 1], 1));
+            const uint32_t pk = odd ? A::pack_hi(got, keep) : A::pack_hi(keep, got);
+            if (j + (odd ? 1 : 0) < rows) *reinterpret_cast<uint32_t*>(yl + j * a.ldy) = pk;
+        }
+    } else if (nn < a.N) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if (j < rows) yb[j * a.ldy + nn] = A::from_f32(__uint_as_float(v[j]));
+    }
+}
+
+// four neighbouring outputs of the gate/up mode: g4 and u4 are the sums, wt the routing weight
+template <typename AT>
+__device__ __forceinline__ void store_swiglu(const GemmArgs& a, const float4& g4, const float4& u4, float wt, int64_t row,
+                                             int64_t n) {
+    using A = Act<AT>;
+    const float gv[4] = {g4.x, g4.y, g4.z, g4.w}, uv[4] = {u4.x, u4.y, u4.z, u4.w};
+    float f[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float g = gv[j], u = uv[j];
+        if (a.lim > 0.f) {
+            g = fminf(g, a.lim);
+            u = fminf(fmaxf(u, -a.lim), a.lim);
+        }
+        f[j] = g / (1.0f + __expf(-g)) * u * wt;
+    }
+    uint16_t* yp = reinterpret_cast<uint16_t*>(a.y) + row * a.ldy + n;
+    if (a.y_vec_ok && n + 4 <= a.N) {
+        *reinterpret_cast<uint2*>(yp) = make_uint2(A::pack_hi(f[0], f[1]), A::pack_hi(f[2], f[3]));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (n + j < a.N) yp[j] = A::from_f32(f[j]);
+    }
+}
+
+// Shape of one CTA of the one-tile form: up to 256 activation rows, four A slots (32 columns = one k-block each).
+template <int BITS> struct GemmCfg {
+    static constexpr int TNMAX = 256, RA = 4, NKG = RA, ACOL = TNMAX, NCOLS = 512;
+    static constexpr int CKB = CodeStage<BITS>::CKB, RB = CodeStage<BITS>::RB, CD = 6;
+    static constexpr int C_STAGE = 128 * RB, X_STAGE = TNMAX * GEMM_BK * 2;
+    static constexpr int NDW = 4 * NKG, THREADS = 128 + 32 * NDW;
+    static constexpr int NBAR = 2 * RA + 2 * CD + 1;
+    static constexpr size_t SMEM = 1024 + (size_t)RA * X_STAGE + (size_t)CD * (C_STAGE + SIDE_SLOT) + NBAR * 8 + 16;
+};
+
+// KS: CTAs of a cluster (along blockIdx.z) that split K, for grids that would leave most SMs idle: every CTA
+// accumulates its share of the k-blocks in its own tensor memory and leaves the sums as float32 in its (by then
+// idle) shared memory; after a cluster barrier CTA r adds and stores the activation rows of its share, in rank order.
+// Both cluster barriers are reached by every thread on every path.
+template <typename AT, int BITS, int KS>
+__global__ void __launch_bounds__(GemmCfg<BITS>::THREADS, 1)
+qgemm_ts_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
+    using A = Act<AT>;
+    using C = GemmCfg<BITS>;
+    constexpr int CKB = C::CKB, RB = C::RB, CD = C::CD, RA = C::RA, NKG = C::NKG;
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // the dynamic shared-memory base is only guaranteed 16-byte aligned: realign to 1024
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* sA = smem;
-    uint8_t* sB = smem + GEMM_SA * A_STAGE;
-    uint8_t* sC = sB + GEMM_SB * B_STAGE;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sC + 2 * C_STAGE);
-    uint64_t* xfull = bars;                  // [SA]
-    uint64_t* xempty = bars + GEMM_SA;       // [SA]
-    uint64_t* bfull = bars + 2 * GEMM_SA;    // [SB]
-    uint64_t* bempty = bfull + GEMM_SB;      // [SB]
-    uint64_t* accfull = bempty + GEMM_SB;    // [1]
+    uint8_t* sX = smem;
+    uint8_t* sC = sX + RA * C::X_STAGE;
+    uint8_t* sSide = sC + CD * C::C_STAGE;
+    uint64_t* full = reinterpret_cast<uint64_t*>(sSide + CD * SIDE_SLOT);     // both operands of a k-block
+    uint64_t* empty = full + RA;
+    uint64_t* cfull = empty + RA;
+    uint64_t* cempty = cfull + CD;
+    uint64_t* accfull = cempty + CD;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accfull + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t n0 = (int64_t)blockIdx.x * BN;
-    int64_t m0 = (int64_t)blockIdx.y * (GEMM_BM * MT), m_end = a.M;
-    const uint32_t* codes_g = a.codes;
-    const void* scales_g = a.scales;
-    const void* biases_g = a.biases;
-    if (a.tile_expert) {
-        // uniform for the whole CTA, before any barrier or tensor-memory allocation
-        if ((int)blockIdx.y >= *a.num_tiles) return;
-        const int e = a.tile_expert[blockIdx.y];
-        if (a.bits_tab && a.bits_tab[e] != BITS) return;
-        m0 = a.tile_row0[blockIdx.y];
-        m_end = a.expert_offsets[e + 1];
-        codes_g = a.codes_tab[e];
-        scales_g = a.scales_tab[e];
-        biases_g = a.biases_tab[e];
-    }
-    // this CTA's k-blocks [kb0, kb1): all of them, or its share (whole code stages) of a split K
+    const int64_t n0 = (int64_t)blockIdx.x * 128;
+    const int64_t m0 = (int64_t)blockIdx.y * a.tn;
+    // activation rows of this tile, and the MMA's N
+    const int rows = (int)min((int64_t)a.tn, a.M - m0);
+    const int n_mma = (rows + 15) & ~15;
+    // this CTA's k-blocks [kb0, kb1): all of them, or its share (whole code stages and sidecar chunks) of a split K
     const int nkb_all = (int)(a.K / GEMM_BK);
     int kb0 = 0, kb1 = nkb_all;
     const int ks_rank = KS > 1 ? (int)blockIdx.z : 0;
     if constexpr (KS > 1) {
-        kb0 = (ks_rank * nkb_all / KS) / CKB * CKB;
-        kb1 = ks_rank == KS - 1 ? nkb_all : ((ks_rank + 1) * nkb_all / KS) / CKB * CKB;
+        kb0 = (ks_rank * nkb_all / KS) / 4 * 4;
+        kb1 = ks_rank == KS - 1 ? nkb_all : ((ks_rank + 1) * nkb_all / KS) / 4 * 4;
     }
-    const int nkb = kb1 - kb0;
+    const int nkb = kb1 - kb0, nst = (nkb + CKB - 1) / CKB;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < GEMM_SA; ++i) { mbar_init(xfull + i, 1); mbar_init(xempty + i, 1); }
-        for (int i = 0; i < GEMM_SB; ++i) { mbar_init(bfull + i, NDW); mbar_init(bempty + i, 1); }
+        for (int i = 0; i < RA; ++i) { mbar_init(full + i, 5); mbar_init(empty + i, 1); }      // 4 dequantizer warps + TMA
+        for (int i = 0; i < CD; ++i) { mbar_init(cfull + i, 64); mbar_init(cempty + i, 4 * CKB); }
         mbar_init(accfull, 1);
         mbar_fence_init();
     }
-    if (warp == 1) tmem_alloc(tmem_slot, MT * BN);
+    if (warp == 1) tmem_alloc(tmem_slot, C::NCOLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -255,321 +259,142 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            for (int lk = 0; lk < nkb && ok; ++lk) {
-                const int s = lk % GEMM_SA;
-                if (lk >= GEMM_SA) ok = mbar_wait(xempty + s, (uint32_t)((lk / GEMM_SA) - 1) & 1u, 1u << 18);
-                if (!ok) break;
-                mbar_expect_tx(xfull + s, A_STAGE);
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt)      // rows past M read as zeros
-                    tma_load_2d(sA + s * A_STAGE + mt * A_TILE, &xmap, (kb0 + lk) * GEMM_BK, (int)m0 + mt * GEMM_BM,
-                                xfull + s);
+        int s = 0;
+        uint32_t ph = 1u;
+        const uint32_t bytes = (uint32_t)(a.tn * GEMM_BK * 2);
+        for (int i = 0; i < nkb; ++i) {
+            ok = __all_sync(0xFFFFFFFFu, ts_wait(empty + s, ph));
+            if (!ok) break;
+            if (elect_one()) {
+                mbar_expect_tx(full + s, bytes);
+                tma_load_2d(sX + s * C::X_STAGE, &xmap, (kb0 + i) * GEMM_BK, (int)m0, full + s);   // rows past M read as zeros
             }
+            __syncwarp();
+            if (++s == RA) { s = 0; ph ^= 1u; }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc<AT, BN>();
-            for (int kb = 0; kb < nkb && ok; ++kb) {      // kb: local index
-                const int s = kb % GEMM_SA, t = kb % GEMM_SB;
-                ok = mbar_wait(xfull + s, (uint32_t)(kb / GEMM_SA) & 1u, 1u << 18) &&
-                     mbar_wait(bfull + t, (uint32_t)(kb / GEMM_SB) & 1u, 1u << 18);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t a_addr = smem_u32(sA + s * A_STAGE), b_addr = smem_u32(sB + t * B_STAGE);
+        const uint32_t idesc = umma_idesc_ts<AT>(n_mma);
+        const uint32_t x_lo = umma_desc_sw128_lo(smem_u32(sX));
+        int s = 0;
+        uint32_t ph = 0u;
+        for (int i = 0; i < nkb; ++i) {
+            ok = __all_sync(0xFFFFFFFFu, ts_wait(full + s, ph));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t xd = x_lo + (uint32_t)s * (uint32_t)(C::X_STAGE >> 4);
+            const uint32_t ac = tmem_base + (uint32_t)(C::ACOL + s * 32);
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < GEMM_BK / 16; ++k)
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt)
-                        umma_f16(tmem_base + (uint32_t)(mt * BN), umma_desc_sw128(a_addr + mt * A_TILE + k * 32),
-                                 umma_desc_sw128(b_addr + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                umma_commit(xempty + s);
-                umma_commit(bempty + t);
+                    umma_f16_ts(tmem_base, ac + k * 8, umma_desc_join(xd + k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                umma_commit(empty + s);
+                if (i == nkb - 1) umma_commit(accfull);
             }
-            if (ok) umma_commit(accfull);
+            __syncwarp();
+            if (++s == RA) { s = 0; ph ^= 1u; }
         }
-    } else {
-        // ---------------- dequantizers: one weight row per thread ----------------
-        const int dt = threadIdx.x - 64;                      // 0 .. NDT-1
-        const int r = dt % BN;                                // row within the tile
-        const int half = dt / BN;                             // DPR = 2: which 32 codes of the k-block (warp-uniform)
-        const int64_t n = min(n0 + r, a.N - 1);               // rows past N are computed but never stored
-        const int64_t rowbytes = a.K * BITS / 8;
-        const uint8_t* cbytes = reinterpret_cast<const uint8_t*>(codes_g);
-        const uint16_t* srow = reinterpret_cast<const uint16_t*>(scales_g) + n * a.G;
-        const uint16_t* brow = reinterpret_cast<const uint16_t*>(biases_g) + n * a.G;
-        const uint32_t row_off = (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u;
-        const uint32_t sw = (uint32_t)(r & 7);
-        const int gs = a.gs;
-        const int st0 = kb0 / CKB, nstage = (kb1 + CKB - 1) / CKB;     // code stages [st0, nstage) (absolute)
-
-        // all dequantizer threads copy code stage `st` together: consecutive lanes take consecutive
-        // 16-byte chunks of a row; always one commit so that group counting stays uniform
-        auto issue_codes = [&](int st, int buf) {
-            if (st < nstage) {
-                const int64_t off = (int64_t)st * RB;
-                const int rem = (int)min((int64_t)RB, rowbytes - off);
-                uint8_t* dstb = sC + buf * C_STAGE;
-                for (int c = dt; c < BN * CPR; c += NDT) {
-                    const int row = c / CPR, col = c - row * CPR;
-                    if (col * 16 < rem)
-                        cp_async16(dstb + row * RBP + (SWZ ? (col ^ swz_of(row)) : col) * 16,
-                                   cbytes + min(n0 + row, a.N - 1) * rowbytes + off + col * 16);
-                }
-            }
-            cp_async_commit();
-        };
-
-        // Scales and biases: one vector load per code stage (CKB consecutive groups of this row) when
-        // the row is suitably aligned and groups are 64 or 128 wide; otherwise scalar loads per k-block.
-        // Either way they are fetched one step ahead of their use.
-        constexpr int SCW = CKB / 2;                          // 32-bit words holding CKB 16-bit sidecars
-        const int gpk_shift = (gs == 128) ? 1 : 0;            // k-blocks per group: 1 (gs 64) or 2 (gs 128)
-        const bool sc_vec = (gs >= 64) && (a.G % (CKB >> gpk_shift) == 0) &&
-                            ((reinterpret_cast<uintptr_t>(srow) | reinterpret_cast<uintptr_t>(brow)) % (2 * CKB) == 0) &&
-                            ((a.G * 2) % (2 * CKB) == 0);
-        uint32_t scw[SCW], bcw[SCW], scn[SCW], bcn[SCW];
-#pragma unroll
-        for (int i = 0; i < SCW; ++i) scw[i] = bcw[i] = scn[i] = bcn[i] = 0u;
-        auto load_sc_stage = [&](int st, uint32_t (&so)[SCW], uint32_t (&bo)[SCW]) {
-            // groups of stage st: first = st*CKB >> gpk_shift, count = CKB >> gpk_shift (a multiple of 2 words when vec)
-            const int gfirst = (st * CKB) >> gpk_shift;
-            const int cnt = CKB >> gpk_shift;
-            if (gfirst + cnt <= a.G) {
-                const uint32_t* sp = reinterpret_cast<const uint32_t*>(srow + gfirst);
-                const uint32_t* bp = reinterpret_cast<const uint32_t*>(brow + gfirst);
-                if (cnt == 8) {
-                    const uint4 sv = __ldg(reinterpret_cast<const uint4*>(sp)), bv = __ldg(reinterpret_cast<const uint4*>(bp));
-                    so[0] = sv.x; if (SCW > 1) so[1 % SCW] = sv.y; if (SCW > 2) { so[2 % SCW] = sv.z; so[3 % SCW] = sv.w; }
-                    bo[0] = bv.x; if (SCW > 1) bo[1 % SCW] = bv.y; if (SCW > 2) { bo[2 % SCW] = bv.z; bo[3 % SCW] = bv.w; }
-                } else if (cnt == 4) {
-                    const uint2 sv = __ldg(reinterpret_cast<const uint2*>(sp)), bv = __ldg(reinterpret_cast<const uint2*>(bp));
-                    so[0] = sv.x; if (SCW > 1) so[1 % SCW] = sv.y;
-                    bo[0] = bv.x; if (SCW > 1) bo[1 % SCW] = bv.y;
-                } else if (cnt == 2) {
-                    so[0] = __ldg(sp); bo[0] = __ldg(bp);
-                } else {                                       // cnt == 1
-                    so[0] = __ldg(srow + gfirst); bo[0] = __ldg(brow + gfirst);
-                }
-            } else {                                           // ragged last stage: element loads
-#pragma unroll
-                for (int i = 0; i < CKB; ++i) {
-                    const int gi = gfirst + i;
-                    if (i < cnt && gi < a.G) {
-                        const uint32_t sv = __ldg(srow + gi), bv = __ldg(brow + gi);
-                        if (i & 1) { so[i / 2] |= sv << 16; bo[i / 2] |= bv << 16; }
-                        else { so[i / 2] = sv; bo[i / 2] = bv; }
-                    }
-                }
-            }
-        };
-        uint16_t s0h = 0, b0h = 0, s1h = 0, b1h = 0, s0n = 0, b0n = 0, s1n = 0, b1n = 0;
-        if (sc_vec) {
-            load_sc_stage(st0, scw, bcw);
-        } else {
-            const int g0 = kb0 * GEMM_BK / gs;
-            s0h = __ldg(srow + g0); b0h = __ldg(brow + g0);
-            s1h = s0h; b1h = b0h;
-            if (gs == 32) { s1h = __ldg(srow + g0 + 1); b1h = __ldg(brow + g0 + 1); }
-        }
-        issue_codes(st0, 0);
-        // After a timed-out wait the warp keeps walking the loops (copies and the named barrier
-        // only), so that no other dequantizer warp is left waiting at the barrier.
-        for (int st = st0; st < nstage; ++st) {
-            cp_async_wait<0>();
-            asm volatile("bar.sync 1, %0;" ::"n"(NDT) : "memory");  // stage st landed; stage st-1 fully consumed
-            issue_codes(st + 1, (st + 1 - st0) & 1);
-            if (sc_vec && st + 1 < nstage) load_sc_stage(st + 1, scn, bcn);
-            const uint8_t* crow = sC + ((st - st0) & 1) * C_STAGE + r * RBP;
-#pragma unroll
-            for (int kbi = 0; kbi < CKB; ++kbi) {
-                const int kb = st * CKB + kbi;             // absolute k-block; lk: its index in this CTA's share
-                if (kb >= kb1) break;
-                const int lk = kb - kb0;
-                const int t = lk % GEMM_SB;
-                uint32_t cur[UW];
-                if constexpr (DPR == 1) {
-                    if constexpr ((8 * BITS) % 16 == 0) {
-                        const uint4* cp = reinterpret_cast<const uint4*>(crow + (SWZ ? 0 : kbi * 8 * BITS));
-#pragma unroll
-                        for (int i = 0; i < UW / 4; ++i) {
-                            const uint4 v = SWZ ? cp[(kbi * (UW / 4) + i) ^ swz_of(r)] : cp[i];
-                            cur[4 * i] = v.x; cur[4 * i + 1] = v.y; cur[4 * i + 2] = v.z; cur[4 * i + 3] = v.w;
-                        }
-                    } else {
-                        const uint2* cp = reinterpret_cast<const uint2*>(crow + kbi * 8 * BITS);
-#pragma unroll
-                        for (int i = 0; i < UW / 2; ++i) {
-                            const uint2 v = cp[i];
-                            cur[2 * i] = v.x; cur[2 * i + 1] = v.y;
-                        }
-                    }
-                } else {
-                    // this thread's 32 codes are BITS whole words; the other half stays zero
-                    auto cword = [&](int off) {      // word at byte `off` of the staged row
-                        const int phys = SWZ ? ((((off >> 4) ^ swz_of(r)) << 4) | (off & 15)) : off;
-                        return *reinterpret_cast<const uint32_t*>(crow + phys);
-                    };
-                    const int off0 = kbi * 8 * BITS + half * BITS * 4;
-#pragma unroll
-                    for (int i = 0; i < UW; ++i) cur[i] = 0u;
-                    if (half == 0) {
-#pragma unroll
-                        for (int i = 0; i < BITS; ++i) cur[i] = cword(off0 + 4 * i);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < BITS; ++i) cur[BITS + i] = cword(off0 + 4 * i);
-                    }
-                }
-                if (sc_vec) {
-                    const int gi = kbi >> gpk_shift;                      // group within the stage (static after unrolling)
-                    const uint32_t swd = scw[gi / 2], bwd = bcw[gi / 2];
-                    s0h = (uint16_t)((gi & 1) ? (swd >> 16) : (swd & 0xFFFFu));
-                    b0h = (uint16_t)((gi & 1) ? (bwd >> 16) : (bwd & 0xFFFFu));
-                    s1h = s0h; b1h = b0h;
-                } else if (kb + 1 < kb1) {        // scalar path: sidecars of the next k-block
-                    const int k1 = (kb + 1) * GEMM_BK;
-                    const int g0 = k1 / gs;
-                    s0n = __ldg(srow + g0); b0n = __ldg(brow + g0);
-                    s1n = s0n; b1n = b0n;
-                    if (gs == 32) { s1n = __ldg(srow + g0 + 1); b1n = __ldg(brow + g0 + 1); }
-                }
-                constexpr int TGTC = (BITS <= A::MANT) ? A::MANT - BITS : 0;
-                constexpr float POST = 1.0f / (float)(1 << TGTC);
-                const float s0 = A::to_f32(s0h), s1 = A::to_f32(s1h), bias0 = A::to_f32(b0h), bias1 = A::to_f32(b1h);
-                // s * 2^-TGT is exact (power-of-two scaling) unless it underflows the 16-bit type
-                const uint32_t sp0 = A::pack_hi(s0 * POST, s0 * POST), sp1 = A::pack_hi(s1 * POST, s1 * POST);
-                const uint32_t bb0 = (uint32_t)b0h * 0x00010001u, bb1 = (uint32_t)b1h * 0x00010001u;
-                if (ok && lk >= GEMM_SB)   // warp-uniform outcome
-                    ok = __all_sync(0xFFFFFFFFu, mbar_wait(bempty + t, (uint32_t)((lk / GEMM_SB) - 1) & 1u, 1u << 18));
-                if (ok) {
-                    uint8_t* dst = sB + t * B_STAGE + row_off;
-#define JQ_CHUNK(C, SP, BB, S, BI) \
-    *reinterpret_cast<uint4*>(dst + (((uint32_t)(C) ^ sw) << 4)) = dequant_chunk<AT, BITS, C>(cur, SP, BB, S, BI);
-                    if (DPR == 1 || half == 0) {
-                        JQ_CHUNK(0, sp0, bb0, s0, bias0) JQ_CHUNK(1, sp0, bb0, s0, bias0)
-                        JQ_CHUNK(2, sp0, bb0, s0, bias0) JQ_CHUNK(3, sp0, bb0, s0, bias0)
-                    }
-                    if (DPR == 1 || half == 1) {
-                        JQ_CHUNK(4, sp1, bb1, s1, bias1) JQ_CHUNK(5, sp1, bb1, s1, bias1)
-                        JQ_CHUNK(6, sp1, bb1, s1, bias1) JQ_CHUNK(7, sp1, bb1, s1, bias1)
-                    }
-#undef JQ_CHUNK
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> tensor-core reads
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bfull + t);
-                }
-                if (!sc_vec) { s0h = s0n; b0h = b0n; s1h = s1n; b1h = b1n; }
-            }
-            if (sc_vec) {
-#pragma unroll
-                for (int i = 0; i < SCW; ++i) { scw[i] = scn[i]; bcw[i] = bcn[i]; }
-            }
-        }
+    } else if (warp < 4) {
+        // ---------------- code loaders ----------------
+        int buf = 0, slot = 0;
+        uint32_t phase = 1u;
+        const SideSrc side = {a.scales, a.biases, nullptr, nullptr, a.G, side_mode(a.scales, a.biases, a.G, a.gs)};
+        ok = load_codes<BITS, 1, CD>(a.codes, n0, a.N, a.K, kb0 / CKB, nst, sC, cfull, cempty, threadIdx.x - 64, buf, phase, side,
+                                     sSide, slot);
+        cp_async_commit();
         cp_async_wait<0>();
-
-        // ---------------- epilogue: TMEM -> registers -> Y ----------------
-        if (ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(accfull, 0, 1u << 18));
-        if constexpr (KS > 1) {
-            // split K: the accumulator is complete, so nothing reads this CTA's stages any more; the CTAs behind
-            // rank 0 leave theirs as float32 rows at the start of their shared memory (rank 0 stores after the
-            // cluster barrier below)
-            if (ok && ks_rank != 0) {
+    } else {
+        // ---------------- dequantizers: one weight row per thread; group kg takes every fourth k-block, A slot kg --------
+        const int quarter = warp & 3, kg = (warp - 4) >> 2;
+        const int r = quarter * 32 + lane;
+        const int64_t n = min(n0 + r, a.N - 1);               // rows past N are computed but never stored
+        const uint32_t a_dst = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(C::ACOL + kg * 32);
+        Sidecars sc;
+        sc.gs = a.gs;
+        sc.mode = side_mode(a.scales, a.biases, a.G, a.gs);
+        sc.row(a.scales, a.biases, n, a.G);
+        if (sc.mode == 0 && kg < nkb) sc.fetch(kb0 + kg);
+        int slot = 0;                                         // chunk ring: this group's k-blocks are in successive chunks
+        uint32_t ph = 1u;
+        int buf = kg / CKB;                                   // ring position, with the parity of the pass on top of it
+        for (int i = kg; i < nst * CKB; i += RA) {
+            const bool odd = buf >= CD;
+            const int cb = odd ? buf - CD : buf;
+            ok = __all_sync(0xFFFFFFFFu, ts_wait(cfull + cb, odd ? 1u : 0u));
+            if (!ok) break;
+            buf += RA / CKB;
+            if (buf >= 2 * CD) buf -= 2 * CD;
+            if (i < nkb) {
+                const int kb = kb0 + i;                        // absolute k-block
+                uint32_t out[32];
+                expand_block<AT, BITS>(sC + cb * C::C_STAGE + r * RB, r, i % CKB, kb, i + RA < nkb ? kb + RA : -1,
+                                       reinterpret_cast<const uint16_t*>(sSide + slot * SIDE_SLOT) + r * 4, sc, out);
+                if (++slot == CD) slot = 0;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(cempty + cb);
+                ok = __all_sync(0xFFFFFFFFu, ts_wait(empty + kg, ph));
+                if (!ok) break;
+                ph ^= 1u;
                 tc_fence_after();
-                const int q = warp & 3, part = (warp - 2) / 4;
-                constexpr int COLS_PER_WARP = BN / (NDW / 4);
-                float* srow_f = reinterpret_cast<float*>(smem) + (size_t)(q * 32 + lane) * KS_PITCH;
-#pragma unroll 1
-                for (int c0 = part * COLS_PER_WARP; c0 < (part + 1) * COLS_PER_WARP; c0 += 32) {
-                    uint32_t v[32];
-                    tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        *reinterpret_cast<float4*>(srow_f + c0 + 4 * j) =
-                            make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                        __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-                }
+                tmem_st32(a_dst, out);
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full + kg);
+            } else if (lane == 0) {                            // the last stage is not always whole
+                mbar_arrive(cempty + cb);
             }
         }
-        if (KS == 1 && ok) {
+
+        // ---------------- epilogue: lane = weight row, TMEM column = activation row ----------------
+        if (ok) ok = __all_sync(0xFFFFFFFFu, ts_wait(accfull, 0));
+        if (ok) {
             tc_fence_after();
-            const int q = warp & 3;                               // TMEM lane quarter this warp may read
-            const int part = (warp - 2) / 4;                      // the NDW/4 warps of a quarter split the columns
-            constexpr int COLS_PER_WARP = BN / (NDW / 4);
+            const uint32_t d_src = tmem_base + ((uint32_t)(quarter * 32) << 16);
+            const int64_t nn = n0 + r;
 #pragma unroll 1
-            for (int mt = 0; mt < MT; ++mt) {
-            const int64_t m = m0 + mt * GEMM_BM + q * 32 + lane;
-            uint16_t* yrow = reinterpret_cast<uint16_t*>(a.y) + m * a.ldy + n0;
-#pragma unroll 1
-            for (int c0 = part * COLS_PER_WARP; c0 < (part + 1) * COLS_PER_WARP; c0 += 32) {
+            for (int c0 = kg * 32; c0 < rows; c0 += NKG * 32) {
                 uint32_t v[32];
-                tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(mt * BN + c0), v);
-                if (m < m_end) {
-                    if (a.y_vec_ok && n0 + c0 + 32 <= a.N) {
+                tmem_ld32(d_src + (uint32_t)c0, v);
+                if constexpr (KS > 1) {
+                    float* part = reinterpret_cast<float*>(smem) + (size_t)c0 * 128 + r;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            uint4 o;
-                            o.x = A::pack_hi(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]));
-                            o.y = A::pack_hi(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]));
-                            o.z = A::pack_hi(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]));
-                            o.w = A::pack_hi(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]));
-                            *reinterpret_cast<uint4*>(yrow + c0 + 8 * j) = o;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (n0 + c0 + j < a.N) yrow[c0 + j] = A::from_f32(__uint_as_float(v[j]));
-                    }
+                    for (int j = 0; j < 32; ++j)
+                        if (c0 + j < rows) part[j * 128] = __uint_as_float(v[j]);
+                } else {
+                    store_columns<AT>(a, v, m0 + c0, rows - c0, nn, n0 + 128 <= a.N, lane);
                 }
-            }
             }
         }
     }
     if constexpr (KS > 1) {
-        static_assert(KS == 1 || (MT == 1 && BN == 256), "split K: one 128 x 256 accumulator per CTA");
-        gemm_cluster_sync();                               // the staged accumulators are complete
-        if (warp >= 2 && ks_rank == 0 && ok) {
-            tc_fence_after();
-            const int q = warp & 3, part = (warp - 2) / 4;
-            constexpr int COLS_PER_WARP = BN / (NDW / 4);
-            const float* srow_f = reinterpret_cast<const float*>(smem) + (size_t)(q * 32 + lane) * KS_PITCH;
-            const int64_t m = m0 + q * 32 + lane;
-            uint16_t* yrow = reinterpret_cast<uint16_t*>(a.y) + m * a.ldy + n0;
-#pragma unroll 1
-            for (int c0 = part * COLS_PER_WARP; c0 < (part + 1) * COLS_PER_WARP; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-                float f[32];
+        static_assert((size_t)C::TNMAX * 128 * 4 <= (size_t)RA * C::X_STAGE + CD * C::C_STAGE, "staged sums fit");
+        ts_cluster_sync();                               // the staged sums are complete
+        if (warp >= 4 && ok) {
+            // CTA r stores activation rows [r, r+1) * rows / KS; a thread adds four neighbouring weight rows
+            const int t0 = ks_rank * rows / KS, t1 = (ks_rank + 1) * rows / KS;
+            constexpr int QPR = 128 / 4;
+            for (int q = threadIdx.x - 128 + t0 * QPR; q < t1 * QPR; q += C::NDW * 32) {
+                const int tok = q / QPR, nl = (q % QPR) * 4;
+                const float* src = reinterpret_cast<const float*>(smem) + (size_t)tok * 128 + nl;
+                float4 f = ld_cluster_f32x4(src, 0);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
                 for (int rk = 1; rk < KS; ++rk) {           // rank order: the same sum whatever the timing
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float4 t = ld_cluster_f32x4(srow_f + c0 + 4 * j, (uint32_t)rk);
-                        f[4 * j] += t.x; f[4 * j + 1] += t.y; f[4 * j + 2] += t.z; f[4 * j + 3] += t.w;
-                    }
+                    const float4 g = ld_cluster_f32x4(src, (uint32_t)rk);
+                    f.x += g.x; f.y += g.y; f.z += g.z; f.w += g.w;
                 }
-                if (m < m_end) {
-                    if (a.y_vec_ok && n0 + c0 + 32 <= a.N) {
+                uint16_t* yp = reinterpret_cast<uint16_t*>(a.y) + (m0 + tok) * a.ldy + n0 + nl;
+                if (a.y_vec_ok && n0 + nl + 4 <= a.N) {
+                    *reinterpret_cast<uint2*>(yp) = make_uint2(A::pack_hi(f.x, f.y), A::pack_hi(f.z, f.w));
+                } else {
+                    const float fv[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            uint4 o;
-                            o.x = A::pack_hi(f[8 * j + 0], f[8 * j + 1]);
-                            o.y = A::pack_hi(f[8 * j + 2], f[8 * j + 3]);
-                            o.z = A::pack_hi(f[8 * j + 4], f[8 * j + 5]);
-                            o.w = A::pack_hi(f[8 * j + 6], f[8 * j + 7]);
-                            *reinterpret_cast<uint4*>(yrow + c0 + 8 * j) = o;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (n0 + c0 + j < a.N) yrow[c0 + j] = A::from_f32(f[j]);
-                    }
+                    for (int j = 0; j < 4; ++j)
+                        if (n0 + nl + j < a.N) yp[j] = A::from_f32(fv[j]);
                 }
             }
         }
-        gemm_cluster_sync();                               // the others keep their shared memory until rank 0 has read it
+        ts_cluster_sync();                               // every CTA keeps its shared memory until all have read it
     }
     if (!ok) atomicOr(a.status, JQ_STATUS_LOCAL_WAIT);
     tc_fence_before();
@@ -580,7 +405,288 @@ qgemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
         if (gave_up)
             for (int i = 0; i < 1000; ++i) __nanosleep(1000);
         tc_fence_after();
-        tmem_dealloc(tmem_base, MT * BN);
+        tmem_dealloc(tmem_base, C::NCOLS);
+    }
+}
+
+// ---- persistent form --------------------------------------------------------------------------------------
+// One CTA per SM walks tiles of 128 weight rows x up to 192 activation rows (blockIdx.x, + gridDim.x, ...).  Two
+// accumulators of 192 columns and four A slots fill the tensor memory: while the epilogue warps store one tile, the
+// MMAs fill the other accumulator, and copies and expansion of the next tile start before this one's MMAs are done.
+// Without it every 128-row tile of an expert paid 5.5 us of start and epilogue for 12 to 64 k-blocks of 0.3 us, and a
+// grid sized for the largest possible tile list started thousands of CTAs that had nothing to do.
+// GU (grouped mode): the tile's 128 weight rows are 64 rows of the gate projection and the same 64 rows of the up
+// projection, so both sums of an output meet in one CTA: the epilogue exchanges them through shared memory in f32 and
+// stores h.  Gate and up results never go through memory, and one launch replaces three.
+template <int BITS> struct PersCfg {
+    static constexpr int TNMAX = 192, ND = 2, RA = 4, NCOLS = 512, NKG = RA;
+    static constexpr int ACOL = ND * TNMAX;
+    static constexpr int CKB = CodeStage<BITS>::CKB, RB = CodeStage<BITS>::RB, CD = 6;
+    static constexpr int C_STAGE = 128 * RB, X_STAGE = TNMAX * GEMM_BK * 2;
+    static constexpr int NDW = 4 * NKG, THREADS = 32 * (8 + NDW);
+    static constexpr int NBAR = 2 * RA + 2 * CD + 2 * ND;
+    static constexpr int SIDE_OFF = RA * X_STAGE + CD * C_STAGE;
+    static constexpr int SW_OFF = SIDE_OFF + CD * SIDE_SLOT;             // float[32][128]: gate/up exchange
+    static constexpr int BAR_OFF = SW_OFF + 32 * 128 * 4;
+    static constexpr size_t SMEM = 1024 + BAR_OFF + NBAR * 8 + 16;
+};
+
+struct PersTile {
+    int64_t n0, m0;
+    int rows;                     // <= 0: nothing to do
+    const uint32_t *codes, *codes2;
+    const void *scales, *biases, *scales2, *biases2;
+};
+
+template <int BITS, bool GU>
+__device__ __forceinline__ PersTile pers_tile(const GemmArgs& a, int tile, int nx) {
+    PersTile t;
+    const int bx = tile % nx, by = tile / nx;
+    t.n0 = (int64_t)bx * (GU ? 64 : 128);
+    const int entry = by / a.sub, part = by - entry * a.sub;
+    const int e = a.tile_expert[entry];
+    t.m0 = (int64_t)a.tile_row0[entry] + (int64_t)part * a.tn;
+    int64_t m_end = a.expert_offsets[e + 1];
+    t.codes = a.codes_tab[e]; t.scales = a.scales_tab[e]; t.biases = a.biases_tab[e];
+    t.codes2 = nullptr; t.scales2 = nullptr; t.biases2 = nullptr;
+    if constexpr (GU) { t.codes2 = a.codes_tab2[e]; t.scales2 = a.scales_tab2[e]; t.biases2 = a.biases_tab2[e]; }
+    if (a.bits_tab && a.bits_tab[e] != BITS) m_end = t.m0;             // a launch of its own width takes it
+    t.rows = (int)min((int64_t)a.tn, m_end - t.m0);
+    return t;
+}
+
+template <bool GU> __device__ __forceinline__ int pers_side_mode(const GemmArgs& a, const PersTile& t) {
+    const int m = side_mode(t.scales, t.biases, a.G, a.gs);
+    if constexpr (!GU) return m;
+    const int m2 = side_mode(t.scales2, t.biases2, a.G, a.gs);
+    return m == 0 || m2 == 0 ? 0 : max(m, m2);               // the copy that both matrices are aligned for
+}
+
+template <typename AT, int BITS, bool GU>
+__global__ void __launch_bounds__(PersCfg<BITS>::THREADS, 1)
+qgemm_pers_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
+    using C = PersCfg<BITS>;
+    constexpr int CKB = C::CKB, RB = C::RB, CD = C::CD, RA = C::RA, NKG = C::NKG;
+
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* sX = smem;
+    uint8_t* sC = sX + RA * C::X_STAGE;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::BAR_OFF);      // both operands of a k-block
+    uint64_t* empty = full + RA;
+    uint64_t* cfull = empty + RA;
+    uint64_t* cempty = cfull + CD;
+    uint64_t* accfull = cempty + CD;
+    uint64_t* accempty = accfull + C::ND;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accempty + C::ND);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nkb = (int)(a.K / GEMM_BK), nst = (nkb + CKB - 1) / CKB;
+    const int nx = (int)((a.N + (GU ? 63 : 127)) / (GU ? 64 : 128));
+    const int total = nx * *a.num_tiles * a.sub;
+    const int first = blockIdx.x, step = gridDim.x;
+    if (first >= total) return;              // uniform for the CTA, before any barrier or tensor-memory allocation
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < RA; ++i) { mbar_init(full + i, 5); mbar_init(empty + i, 1); }      // 4 dequantizer warps + TMA
+        for (int i = 0; i < CD; ++i) { mbar_init(cfull + i, 64); mbar_init(cempty + i, 4 * CKB); }      // every k-block of a stage has its group
+        for (int i = 0; i < C::ND; ++i) { mbar_init(accfull + i, 1); mbar_init(accempty + i, 4); }
+        mbar_fence_init();
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, C::NCOLS);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    bool ok = true;
+    // every wait on an "empty" barrier starts at parity 1: a fresh barrier counts as released.  Each role looks the next
+    // tile up while it works on this one (in grouped mode that is a chain of dependent loads).
+    PersTile next = pers_tile<BITS, GU>(a, first, nx);
+    auto take = [&](int tile) {
+        const PersTile cur = next;
+        if (tile + step < total) next = pers_tile<BITS, GU>(a, tile + step, nx);
+        return cur;
+    };
+
+    if (warp == 0) {
+        // ---------------- TMA producer ----------------
+        int s = 0;
+        uint32_t ph = 1u;
+        for (int tile = first; tile < total && ok; tile += step) {
+            const PersTile t = take(tile);
+            if (t.rows <= 0) continue;
+            const int boxes = (((t.rows + 15) & ~15) + a.box_rows - 1) / a.box_rows;
+            const uint32_t box_bytes = (uint32_t)(a.box_rows * GEMM_BK * 2), bytes = (uint32_t)boxes * box_bytes;
+            for (int i = 0; i < nkb; ++i) {
+                ok = __all_sync(0xFFFFFFFFu, ts_wait(empty + s, ph));
+                if (!ok) break;
+                if (elect_one()) {
+                    mbar_expect_tx(full + s, bytes);
+                    for (int b = 0; b < boxes; ++b)          // rows past M read as zeros
+                        tma_load_2d(sX + s * C::X_STAGE + b * box_bytes, &xmap, i * GEMM_BK, (int)t.m0 + b * a.box_rows,
+                                    full + s);
+                }
+                __syncwarp();
+                if (++s == RA) { s = 0; ph ^= 1u; }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer ----------------
+        const uint32_t x_lo = umma_desc_sw128_lo(smem_u32(sX));
+        int s = 0, d = 0;
+        uint32_t ph = 0u, dph = 1u;
+        for (int tile = first; tile < total && ok; tile += step) {
+            const PersTile t = take(tile);
+            if (t.rows <= 0) continue;
+            const uint32_t idesc = umma_idesc_ts<AT>((t.rows + 15) & ~15);
+            const uint32_t dcol = tmem_base + (uint32_t)(d * C::TNMAX);
+            ok = __all_sync(0xFFFFFFFFu, ts_wait(accempty + d, dph));
+            for (int i = 0; i < nkb && ok; ++i) {
+                ok = __all_sync(0xFFFFFFFFu, ts_wait(full + s, ph));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t xd = x_lo + (uint32_t)s * (uint32_t)(C::X_STAGE >> 4);
+                const uint32_t ac = tmem_base + (uint32_t)(C::ACOL + s * 32);
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < GEMM_BK / 16; ++k)
+                        umma_f16_ts(dcol, ac + k * 8, umma_desc_join(xd + k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(empty + s);
+                    if (i == nkb - 1) umma_commit(accfull + d);
+                }
+                __syncwarp();
+                if (++s == RA) { s = 0; ph ^= 1u; }
+            }
+            if (++d == C::ND) { d = 0; dph ^= 1u; }
+        }
+    } else if (warp < 4) {
+        // ---------------- code loaders ----------------
+        int buf = 0, slot = 0;
+        uint32_t ph = 1u;
+        for (int tile = first; tile < total && ok; tile += step) {
+            const PersTile t = take(tile);
+            if (t.rows <= 0) continue;
+            const SideSrc side = {t.scales, t.biases, t.scales2, t.biases2, a.G, pers_side_mode<GU>(a, t)};
+            ok = load_codes<BITS, 1, CD, GU>(t.codes, t.n0, a.N, a.K, 0, nst, sC, cfull, cempty, threadIdx.x - 64, buf, ph, side,
+                                             smem + C::SIDE_OFF, slot, t.codes2);
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+    } else if (warp < 8) {
+        // ---------------- epilogue: lane = weight row, TMEM column = activation row ----------------
+        const int quarter = warp & 3, r = quarter * 32 + lane;
+        int d = 0;
+        uint32_t dph = 0u;
+        for (int tile = first; tile < total && ok; tile += step) {
+            const PersTile t = take(tile);
+            if (t.rows <= 0) continue;
+            ok = __all_sync(0xFFFFFFFFu, ts_wait(accfull + d, dph));
+            if constexpr (GU) {      // the four warps meet in barriers below: they go on or leave together
+                int all;
+                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+                             "barrier.cta.red.and.aligned.pred q, 1, 128, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+                             : "=r"(all) : "r"(ok ? 1 : 0) : "memory");
+                ok = all != 0;
+            }
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t src = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(d * C::TNMAX);
+#pragma unroll 1
+            for (int c0 = 0; c0 < t.rows; c0 += 32) {
+                uint32_t v[32];
+                tmem_ld32(src + (uint32_t)c0, v);
+                if (c0 + 32 >= t.rows) {                     // the accumulator is read: the MMAs may have it back
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(accempty + d);
+                }
+                if constexpr (GU) {
+                    float* sw = reinterpret_cast<float*>(smem + C::SW_OFF);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sw[j * 128 + r] = __uint_as_float(v[j]);
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    const int nrow = min(32, t.rows - c0);
+                    for (int q = r; q < nrow * 16; q += 128) {
+                        const int tok = q >> 4, nl = (q & 15) * 4;
+                        const float4 g4 = *reinterpret_cast<const float4*>(sw + tok * 128 + nl);
+                        const float4 u4 = *reinterpret_cast<const float4*>(sw + tok * 128 + 64 + nl);
+                        const int64_t row = t.m0 + c0 + tok;
+                        const float wt = a.wts ? a.wts[a.order[row]] : 1.0f;
+                        store_swiglu<AT>(a, g4, u4, wt, row, t.n0 + nl);
+                    }
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                } else {
+                    store_columns<AT>(a, v, t.m0 + c0, t.rows - c0, t.n0 + r, t.n0 + 128 <= a.N, lane);
+                }
+            }
+            if (++d == C::ND) { d = 0; dph ^= 1u; }
+        }
+    } else {
+        // ---------------- dequantizers: one weight row per thread, alternate k-blocks per group ----------------
+        const int quarter = warp & 3, kg = (warp - 8) >> 2, r = quarter * 32 + lane;
+        const uint32_t a_dst = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)C::ACOL;
+        const bool up = GU && r >= 64;                        // warp-uniform
+        auto row_of = [&](const PersTile& t) { return min(t.n0 + (GU ? r & 63 : r), a.N - 1); };   // past N: computed, never stored
+        Sidecars sc;
+        sc.gs = a.gs;
+        int slot0 = 0;                                        // sidecar ring: slot of the tile's first chunk
+        // k-block g of this CTA (counted over all its tiles) belongs to group g % 4 and to A slot g % 4; the codes are in
+        // stages of CKB k-blocks, each of another group, counted over all tiles as well
+        uint32_t ph = 1u;
+        int base = 0, sbase = 0;                              // k-blocks (mod 4) and stages (mod 2 CD) before this tile
+        for (int tile = first; tile < total && ok; tile += step) {
+            const PersTile t = take(tile);
+            if (t.rows <= 0) continue;
+            int kb = (kg - base) & 3;
+            int buf = sbase + kb / CKB;                       // ring position, with the parity of the pass on top of it
+            if (buf >= 2 * CD) buf -= 2 * CD;
+            int slot = slot0;                                 // this group's k-blocks are in successive chunks
+            sc.mode = pers_side_mode<GU>(a, t);
+            sc.row(up ? t.scales2 : t.scales, up ? t.biases2 : t.biases, row_of(t), a.G);
+            if (sc.mode == 0 && kb < nkb) sc.fetch(kb);
+            for (; kb < nst * CKB; kb += RA) {
+                const bool odd = buf >= CD;
+                const int cb = odd ? buf - CD : buf;
+                ok = __all_sync(0xFFFFFFFFu, ts_wait(cfull + cb, odd ? 1u : 0u));
+                if (!ok) break;
+                buf += RA / CKB;
+                if (buf >= 2 * CD) buf -= 2 * CD;
+                if (kb < nkb) {
+                    uint32_t out[32];
+                    expand_block<AT, BITS>(sC + cb * C::C_STAGE + r * RB, r, kb % CKB, kb, kb + RA < nkb ? kb + RA : -1,
+                                           reinterpret_cast<const uint16_t*>(smem + C::SIDE_OFF + slot * SIDE_SLOT) + r * 4, sc,
+                                           out);
+                    if (++slot == CD) slot = 0;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(cempty + cb);
+                    ok = __all_sync(0xFFFFFFFFu, ts_wait(empty + kg, ph));
+                    if (!ok) break;
+                    ph ^= 1u;
+                    tc_fence_after();
+                    tmem_st32(a_dst + (uint32_t)(kg * 32), out);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full + kg);
+                } else if (lane == 0) {                       // the last stage of a tile is not always whole
+                    mbar_arrive(cempty + cb);
+                }
+            }
+            base = (base + nkb) & 3;
+            sbase = (sbase + nst) % (2 * CD);
+            slot0 = (slot0 + (nkb + 3) / 4) % CD;
+        }
+    }
+    if (!ok) atomicOr(a.status, JQ_STATUS_LOCAL_WAIT);
+    tc_fence_before();
+    const int gave_up = __syncthreads_or(ok ? 0 : 1);
+    if (warp == 1) {
+        // after a wait that gave up, copies and MMAs of this CTA may still be in flight: give them a millisecond
+        // to land before the tensor memory goes back and the CTA's shared memory is reused
+        if (gave_up)
+            for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+        tc_fence_after();
+        tmem_dealloc(tmem_base, C::NCOLS);
     }
 }
 
@@ -598,26 +704,24 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// m_tiles: 128-row tiles of a dense GEMM (MT of them per CTA), or entries of a grouped GEMM's tile list (one CTA
-// each, whatever MT)
-template <typename AT, int BITS, int BN, int DPR, int MT = 1, int KS = 1>
+template <typename AT, int BITS, int KS>
 static int launch_gemm(const CUtensorMap& xmap, const GemmArgs& a, int64_t m_tiles, cudaStream_t st) {
-    constexpr size_t smem = CodeStage<BITS, BN, MT>::SMEM;
+    using C = GemmCfg<BITS>;
+    constexpr size_t smem = C::SMEM;
     static_assert(smem <= GEMM_SMEM, "shared memory of one CTA");
-    static_assert(KS == 1 || 1024 + 128 * KS_PITCH * sizeof(float) <= smem - 512, "staged accumulator fits the stages");
+    auto kernel = qgemm_ts_kernel<AT, BITS, KS>;
     static bool attr_done[64] = {};
     int dev = 0;
     JQ_CUDA_OK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_done[dev]) {
-        JQ_CUDA_OK(cudaFuncSetAttribute(qgemm_tc_kernel<AT, BITS, BN, DPR, MT, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
+        JQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (dev >= 0 && dev < 64) attr_done[dev] = true;
     }
-    dim3 grid((unsigned)((a.N + BN - 1) / BN), (unsigned)(a.tile_expert ? m_tiles : (m_tiles + MT - 1) / MT), KS);
+    dim3 grid((unsigned)((a.N + 127) / 128), (unsigned)m_tiles, KS);
     if constexpr (KS > 1) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid;
-        cfg.blockDim = dim3(64 + BN * DPR);
+        cfg.blockDim = dim3(C::THREADS);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
@@ -625,10 +729,29 @@ static int launch_gemm(const CUtensorMap& xmap, const GemmArgs& a, int64_t m_til
         attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = KS;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        JQ_CUDA_OK(cudaLaunchKernelEx(&cfg, qgemm_tc_kernel<AT, BITS, BN, DPR, MT, KS>, xmap, a));
+        JQ_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, xmap, a));
         return JQ_OK;
     }
-    qgemm_tc_kernel<AT, BITS, BN, DPR, MT, KS><<<grid, 64 + BN * DPR, smem, st>>>(xmap, a);
+    kernel<<<grid, C::THREADS, smem, st>>>(xmap, a);
+    return check_launch("qgemm");
+}
+
+template <typename AT, int BITS, bool GU>
+static int launch_pers(const CUtensorMap& xmap, const GemmArgs& a, int64_t m_tiles, cudaStream_t st) {
+    using C = PersCfg<BITS>;
+    static_assert(C::SMEM <= GEMM_SMEM, "shared memory of one CTA");
+    auto kernel = qgemm_pers_kernel<AT, BITS, GU>;
+    static bool attr_done[64] = {};
+    int dev = 0;
+    JQ_CUDA_OK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !attr_done[dev]) {
+        JQ_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
+        if (dev >= 0 && dev < 64) attr_done[dev] = true;
+    }
+    const int64_t nx = (a.N + (GU ? 63 : 127)) / (GU ? 64 : 128), tiles = nx * m_tiles;
+    JQ_REQUIRE(tiles < (1ll << 31), JQ_EUNSUPPORTED, "too many tiles for one launch (%lld)", (long long)tiles);
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, sm_count());
+    kernel<<<grid, C::THREADS, C::SMEM, st>>>(xmap, a);
     return check_launch("qgemm");
 }
 
@@ -638,7 +761,14 @@ struct GroupedArgs {
     const void* const* scales_tab;
     const void* const* biases_tab;
     int64_t max_tiles;
-    int tile_m;       // rows per entry of the tile list: 128, or 256 (two accumulators per CTA)
+    int tile_m;       // rows per entry of the tile list: 128, 192 or 256
+    // gate/up mode: the up projection's tables and what the epilogue needs (GemmArgs)
+    const uint32_t* const* codes_tab2 = nullptr;
+    const void* const* scales_tab2 = nullptr;
+    const void* const* biases_tab2 = nullptr;
+    const float* wts = nullptr;
+    const int32_t* order = nullptr;
+    float lim = 0.f;
 };
 
 // Dense when grp == nullptr (codes/scales/biases of one matrix); grouped otherwise (x holds the M
@@ -666,21 +796,11 @@ int qgemm_dispatch(const void* x, int x_dtype, int64_t M, int64_t ldx, const uin
     EncodeTiledFn enc = encode_tiled_fn();
     JQ_REQUIRE(enc != nullptr, JQ_ECUDA, "cuTensorMapEncodeTiled is not available from this driver");
 
-    CUtensorMap xmap;
-    const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
-    const cuuint64_t gstride[1] = {(cuuint64_t)ldx * 2};
-    const cuuint32_t box[2] = {GEMM_BK, GEMM_BM};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult cr = enc(&xmap, x_dtype == JQ_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-                      const_cast<void*>(x), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    JQ_REQUIRE(cr == CUDA_SUCCESS, JQ_ECUDA, "cuTensorMapEncodeTiled failed with code %d", (int)cr);
-
     GemmArgs a;
     a.codes = codes; a.scales = scales; a.biases = biases; a.y = y;
     a.M = M; a.N = N; a.K = K; a.ldy = ldy; a.gs = gs; a.G = (int)(K / gs);
-    a.y_vec_ok = (aligned(y, 16) && ldy % 8 == 0) ? 1 : 0;
+    a.y_pair_ok = (aligned(y, 4) && ldy % 2 == 0) ? 1 : 0;
+    a.y_vec_ok = (aligned(y, 8) && ldy % 4 == 0) ? 1 : 0;
     a.status = status_word();
     JQ_REQUIRE(a.status != nullptr, JQ_ECUDA, "could not locate the device status word");
     a.tile_expert = grp ? grp->tile_expert : nullptr;
@@ -691,49 +811,77 @@ int qgemm_dispatch(const void* x, int x_dtype, int64_t M, int64_t ldx, const uin
     a.scales_tab = grp ? grp->scales_tab : nullptr;
     a.biases_tab = grp ? grp->biases_tab : nullptr;
     a.bits_tab = grp ? grp->bits_tab : nullptr;
-    const int64_t m_tiles = grp ? grp->max_tiles : (M + GEMM_BM - 1) / GEMM_BM;
-    if (m_tiles == 0) return JQ_OK;
-    JQ_REQUIRE(m_tiles < 65536, JQ_EUNSUPPORTED, "too many row tiles for one launch (%lld)", (long long)m_tiles);
-    // 256-wide tiles reuse every activation tile twice as often; narrow outputs keep 128.  Two row tiles per CTA
-    // (dense only: the grouped tile lists are per 128 rows) when that still leaves a CTA for most SMs.
-    const bool wide = N >= 256;
-    JQ_REQUIRE(!grp || grp->tile_m == 128 || (grp->tile_m == 256 && wide && x_dtype == JQ_BF16), JQ_EUNSUPPORTED,
-               "tile lists of 256 rows need bf16 activations and N >= 256 (128 otherwise)");
-    // Dense GEMMs pick the form with the shortest estimated time.  A CTA walks a k-block in about 1.1 us with one
-    // accumulator and 1.3 us with two (measured; the dequantizer warps set the pace), whatever the grid, so what
-    // counts is the number of waves and the k-blocks per CTA:
-    //   one accumulator            waves(tiles)      * nkb * 1.1
-    //   two accumulators (MT = 2)  waves(tiles / 2)  * nkb * 1.3     (every weight tile dequantized once for two)
-    //   split K over S CTAs        waves(tiles * S)  * (nkb / S * 1.1 + 8)   (8 us: staging and adding the accumulators)
-    bool two = grp ? grp->tile_m == 256 : false;
-    int ksplit = 1;
-    if (!grp && wide && x_dtype == JQ_BF16) {
-        const int64_t sms = sm_count(), ncol = (N + 255) / 256, nkb_all = K / GEMM_BK;
-        auto waves = [&](int64_t ctas) { return (double)((ctas + sms - 1) / sms); };
-        double best = waves(ncol * m_tiles) * nkb_all * 1.1;
-        if (m_tiles >= 2) {
-            const double t2 = waves(ncol * ((m_tiles + 1) / 2)) * nkb_all * 1.3;
-            if (t2 < best) { best = t2; two = true; }
+    const bool gu = grp && grp->codes_tab2;
+    a.codes_tab2 = gu ? grp->codes_tab2 : nullptr;
+    a.scales_tab2 = gu ? grp->scales_tab2 : nullptr;
+    a.biases_tab2 = gu ? grp->biases_tab2 : nullptr;
+    a.wts = gu ? grp->wts : nullptr;
+    a.order = gu ? grp->order : nullptr;
+    a.lim = gu ? grp->lim : 0.f;
+    int ks = 1;
+    int64_t m_tiles;
+    if (grp) {
+        JQ_REQUIRE(grp->tile_m == 128 || grp->tile_m == 192 || (grp->tile_m == 256 && N >= 256 && x_dtype == JQ_BF16),
+                   JQ_EUNSUPPORTED, "tile lists of 256 rows need bf16 activations and N >= 256 (128 or 192 otherwise)");
+        a.tn = grp->tile_m == 192 ? 192 : 128;
+        a.sub = grp->tile_m / a.tn;
+        a.box_rows = 32;
+        m_tiles = grp->max_tiles * a.sub;
+    } else {
+        // The number of row tiles (nt, of tn rows each) and the K split with the shortest estimated time.  Measured on
+        // B200 over M = 17 .. 4096: a CTA walks a k-block in 0.20 + 0.0006 tn us (the expansion of the codes sets the
+        // pace below some 150 rows, the MMAs above) and spends 5.5 us on its start, first copies and epilogue; a split
+        // adds 1.5 us + 8 ns per row for the exchange of the sums.  One CTA per SM, so what counts is the number of waves.
+        // Examples (us): 61 rows, 4096x4096 6-bit: 12.2 split by 4, 15.9 by 2, 27 unsplit; 512 rows, 11008x4096 2-bit:
+        // 50.1 with three tiles of 176, 53.3 with two of 256, 66.6 with four of 128.
+        const int64_t sms = sm_count(), ncol = (N + 127) / 128, nkb_all = K / GEMM_BK;
+        const int64_t least = (M + 255) / 256;
+        m_tiles = least;
+        a.tn = 256;
+        double best = 1e30;
+        for (int64_t nt = least; nt <= least + 3; ++nt) {
+            const int64_t tn = ((M + nt - 1) / nt + 15) / 16 * 16, tiles = (M + tn - 1) / tn;
+            for (int S : {1, 2, 4}) {
+                if (S > 1 && nkb_all / S < 8) continue;
+                const int64_t slots = sms / S * S, ctas = ncol * tiles * S;
+                const double t = (double)((ctas + slots - 1) / slots) *
+                                 ((double)nkb_all / S * (0.20 + 0.0006 * tn) + 5.5 + (S > 1 ? 1.5 + 0.008 * tn : 0.0));
+                if (t < best) { best = t; m_tiles = tiles; a.tn = (int)tn; ks = S; }
+            }
         }
-        for (int S : {2, 4}) {      // clusters of 8 such CTAs were measured at half the speed of 4 (72.9 vs 33.9 us)
-            if (nkb_all / S < 16) continue;
-            const double ts = waves(ncol * m_tiles * S) * ((double)nkb_all / S * 1.1 + 8.0);
-            if (ts < best) { best = ts; two = false; ksplit = S; }
-        }
+        a.sub = 1;
+        a.box_rows = a.tn;
     }
-#define JQ_GEMM_CASE(B)                                                                                  \
-    if (bits == B) {                                                                                     \
-        if (x_dtype == JQ_BF16) {                                                                        \
-            if (two) return launch_gemm<__nv_bfloat16, B, 256, 1, 2>(xmap, a, m_tiles, st);              \
-            if (ksplit == 4) return launch_gemm<__nv_bfloat16, B, 256, 1, 1, 4>(xmap, a, m_tiles, st);  \
-            if (ksplit == 2) return launch_gemm<__nv_bfloat16, B, 256, 1, 1, 2>(xmap, a, m_tiles, st);  \
-            return wide ? launch_gemm<__nv_bfloat16, B, 256, 1>(xmap, a, m_tiles, st)                    \
-                        : launch_gemm<__nv_bfloat16, B, 128, 1>(xmap, a, m_tiles, st);                   \
-        }                                                                                                \
-        return launch_gemm<__half, B, 128, 1>(xmap, a, m_tiles, st);                                     \
+    if (m_tiles == 0) return JQ_OK;
+    JQ_REQUIRE((grp ? grp->max_tiles : (M + GEMM_BM - 1) / GEMM_BM) < 65536, JQ_EUNSUPPORTED,
+               "too many row tiles for one launch (%lld)", (long long)(grp ? grp->max_tiles : (M + GEMM_BM - 1) / GEMM_BM));
+    CUtensorMap xmap;
+    const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
+    const cuuint64_t gstride[1] = {(cuuint64_t)ldx * 2};
+    const cuuint32_t box[2] = {GEMM_BK, (cuuint32_t)a.box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    CUresult cr = enc(&xmap, x_dtype == JQ_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+                      const_cast<void*>(x), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    JQ_REQUIRE(cr == CUDA_SUCCESS, JQ_ECUDA, "cuTensorMapEncodeTiled failed with code %d", (int)cr);
+
+#define JQ_GEMM_T(T, B)                                                                                   \
+    {                                                                                                     \
+        if (gu) return launch_pers<T, B, true>(xmap, a, m_tiles, st);                                     \
+        if (grp) return launch_pers<T, B, false>(xmap, a, m_tiles, st);                              \
+        if (ks == 4) return launch_gemm<T, B, 4>(xmap, a, m_tiles, st);                                   \
+        if (ks == 2) return launch_gemm<T, B, 2>(xmap, a, m_tiles, st);                                   \
+        return launch_gemm<T, B, 1>(xmap, a, m_tiles, st);                                                \
+    }
+#define JQ_GEMM_CASE(B)                                                                                   \
+    if (bits == B) {                                                                                      \
+        if (x_dtype == JQ_BF16) JQ_GEMM_T(__nv_bfloat16, B)                                               \
+        JQ_GEMM_T(__half, B)                                                                              \
     }
     JQ_GEMM_CASE(2) JQ_GEMM_CASE(3) JQ_GEMM_CASE(4) JQ_GEMM_CASE(5) JQ_GEMM_CASE(6) JQ_GEMM_CASE(8)
 #undef JQ_GEMM_CASE
+#undef JQ_GEMM_T
     return fail(JQ_EUNSUPPORTED, "bits=%d", bits);
 }
 
@@ -863,7 +1011,7 @@ int jq_moe_gemm_tiled(const void* x_sorted, int act_dtype, int64_t max_rows, int
                       const void* const* biases_tab, const int32_t* bits_tab, int sidecar_dtype, int64_t N, int64_t K,
                       int bits, int group_size, void* y_sorted, int64_t ldy, jq_stream_t stream) {
     using namespace jq;
-    JQ_REQUIRE(tile_m == 128 || tile_m == 256, JQ_EINVAL, "tile_m must be 128 or 256");
+    JQ_REQUIRE(tile_m == 128 || tile_m == 192 || tile_m == 256, JQ_EINVAL, "tile_m must be 128, 192 or 256");
     JQ_REQUIRE(expert_offsets && tile_expert && tile_row0 && num_tiles && codes_tab && scales_tab && biases_tab,
                JQ_EINVAL, "null pointer");
     JQ_REQUIRE(max_tiles >= 0, JQ_EINVAL, "negative max_tiles");
@@ -874,6 +1022,30 @@ int jq_moe_gemm_tiled(const void* x_sorted, int act_dtype, int64_t max_rows, int
     g.tile_m = tile_m;
     return qgemm_dispatch(x_sorted, act_dtype, max_rows, ldx, nullptr, nullptr, nullptr, sidecar_dtype, N, K, bits,
                           group_size, y_sorted, act_dtype, ldy, &g, (cudaStream_t)stream);
+}
+
+int jq_moe_gate_up_swiglu(const void* x_sorted, int act_dtype, int64_t max_rows, int64_t ldx,
+                          const int32_t* expert_offsets, const int32_t* tile_expert, const int32_t* tile_row0,
+                          const int32_t* num_tiles, int64_t max_tiles, int tile_m, const uint32_t* const* gate_codes,
+                          const void* const* gate_scales, const void* const* gate_biases,
+                          const uint32_t* const* up_codes, const void* const* up_scales, const void* const* up_biases,
+                          int sidecar_dtype, int64_t N, int64_t K, int bits, int group_size, const float* weights,
+                          const int32_t* order, float limit, void* h, int64_t ldh, jq_stream_t stream) {
+    using namespace jq;
+    JQ_REQUIRE(tile_m == 128 || tile_m == 192 || tile_m == 256, JQ_EINVAL, "tile_m must be 128, 192 or 256");
+    JQ_REQUIRE(expert_offsets && tile_expert && tile_row0 && num_tiles && gate_codes && gate_scales && gate_biases &&
+               up_codes && up_scales && up_biases, JQ_EINVAL, "null pointer");
+    JQ_REQUIRE(weights == nullptr || order != nullptr, JQ_EINVAL, "routing weights need the sort order");
+    JQ_REQUIRE(max_tiles >= 0, JQ_EINVAL, "negative max_tiles");
+    GroupedArgs g;
+    g.tile_expert = tile_expert; g.tile_row0 = tile_row0; g.num_tiles = num_tiles; g.expert_offsets = expert_offsets;
+    g.bits_tab = nullptr; g.codes_tab = gate_codes; g.scales_tab = gate_scales; g.biases_tab = gate_biases;
+    g.max_tiles = max_tiles;
+    g.tile_m = tile_m;
+    g.codes_tab2 = up_codes; g.scales_tab2 = up_scales; g.biases_tab2 = up_biases;
+    g.wts = weights; g.order = order; g.lim = limit;
+    return qgemm_dispatch(x_sorted, act_dtype, max_rows, ldx, nullptr, nullptr, nullptr, sidecar_dtype, N, K, bits,
+                          group_size, h, act_dtype, ldh, &g, (cudaStream_t)stream);
 }
 
 }  // extern "C"

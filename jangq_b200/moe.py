@@ -177,13 +177,16 @@ def _gather_qgemv(x: torch.Tensor, x_div: int, pair_expert: torch.Tensor, bank: 
     return y
 
 
+def _same_shape(a: ExpertBank, b: ExpertBank) -> bool:
+    """Two banks of equal shape and one common width: one launch can take both."""
+    return (a.N == b.N and a.K == b.K and a.group_size == b.group_size and a.E == b.E and a.bits_tab is None and
+            b.bits_tab is None and a.distinct_bits == b.distinct_bits and len(a.distinct_bits) == 1)
+
+
 def _gather_qgemv_pair(x: torch.Tensor, x_div: int, pair_expert: torch.Tensor, bank_a: ExpertBank, bank_b: ExpertBank,
                        flags: int = 0, expert_base: int = 0):
     """Two banks of equal shape and width (gate, up) over the same rows of x in one launch."""
-    same = (bank_a.N == bank_b.N and bank_a.K == bank_b.K and bank_a.group_size == bank_b.group_size and
-            bank_a.E == bank_b.E and bank_a.bits_tab is None and bank_b.bits_tab is None and
-            bank_a.distinct_bits == bank_b.distinct_bits and len(bank_a.distinct_bits) == 1)
-    if not same:
+    if not _same_shape(bank_a, bank_b):
         return (_gather_qgemv(x, x_div, pair_expert, bank_a, flags, expert_base),
                 _gather_qgemv(x, x_div, pair_expert, bank_b, flags, expert_base))
     lib = _lib.load()
@@ -408,16 +411,23 @@ def moe_layer(x: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, gate: ExpertB
     with torch.cuda.device(dev):
         use_sorted = P >= SORT_THRESHOLD if few_token_path is None else not few_token_path
         if use_sorted and gate.gemm_ok and up.gemm_ok and down.gemm_ok:
-            # experts with at least 256 rows on average: 256-row tiles, two accumulators per CTA share every
-            # dequantized weight tile (bf16, all three projections at least 256 wide)
-            big = (x.dtype == torch.bfloat16 and min(gate.N, up.N, down.N) >= 256 and P >= 256 * gate.E)
-            sp = SortedPairs(idx32, gate.E, expert_base, tile_m=256 if big else 128)
+            # the grouped kernels take up to 192 rows of an expert per tile, and as many MMA columns as there are rows
+            sp = SortedPairs(idx32, gate.E, expert_base, tile_m=_lib.MOE_GEMM_TILE_M)
             xs = _gather_rows(x, sp, k)
-            g = _moe_gemm(xs, sp, gate)
-            u = _moe_gemm(xs, sp, up)
             h = torch.empty((max(P, 1), I), dtype=x.dtype, device=dev)
-            _lib.check(lib.jq_moe_swiglu(g.data_ptr(), u.data_ptr(), g.stride(0), wf.data_ptr(), sp.order.data_ptr(),
-                                         sp.count_ptr, h.data_ptr(), h.stride(0), I, P, float(swiglu_limit), dt, st))
+            if _same_shape(gate, up):
+                ga, ua = gate._sidecars_as(x.dtype), up._sidecars_as(x.dtype)
+                _lib.check(lib.jq_moe_gate_up_swiglu(
+                    xs.data_ptr(), dt, sp.n, xs.stride(0), sp.offsets.data_ptr(), sp.tile_expert.data_ptr(),
+                    sp.tile_row0.data_ptr(), sp.num_tiles.data_ptr(), sp.max_tiles, sp.tile_m, ga.codes_tab.data_ptr(),
+                    ga.scales_tab.data_ptr(), ga.biases_tab.data_ptr(), ua.codes_tab.data_ptr(), ua.scales_tab.data_ptr(),
+                    ua.biases_tab.data_ptr(), dt, ga.N, ga.K, ga.distinct_bits[0], ga.group_size, wf.data_ptr(),
+                    sp.order.data_ptr(), float(swiglu_limit), h.data_ptr(), h.stride(0), st))
+            else:
+                g = _moe_gemm(xs, sp, gate)
+                u = _moe_gemm(xs, sp, up)
+                _lib.check(lib.jq_moe_swiglu(g.data_ptr(), u.data_ptr(), g.stride(0), wf.data_ptr(), sp.order.data_ptr(),
+                                             sp.count_ptr, h.data_ptr(), h.stride(0), I, P, float(swiglu_limit), dt, st))
             y = _moe_gemm(h, sp, down)
             inv_ptr = sp.inv.data_ptr()
         else:

@@ -702,3 +702,50 @@ def test_swiglu_gather_of_many_pairs_few_of_them_local(P, E, base, E_all):
     close(y.float().cpu().numpy(), want)
     assert torch.count_nonzero(y[torch.from_numpy(~local).to(DEV)]) == 0
     _lib.check(lib.jq_device_status())
+
+
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
+@pytest.mark.parametrize("bits,K,N,gs", ((2, 256, 128, 64), (4, 384, 72, 64), (3, 384, 200, 128), (8, 192, 64, 64), (6, 128, 100, 32)))
+def test_gate_up_swiglu_in_one_launch(bits, K, N, gs, dtype):
+    """jq_moe_gate_up_swiglu against float64 over the same rounded weights: experts of 0, 1, 16, 17, 128, 129, 192 and 193
+    rows (MMA columns, tiles of 192), ragged N (72, 200, 100), sidecars staged and not, clamp and routing weights.
+    Bound: one rounding of h to 16 bits plus the float32 sums (1e-3 of the largest |h|, as in the GEMM tests)."""
+    from jangq_b200 import moe
+    lib = _lib.load()
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(bits + K)
+    counts = (0, 1, 16, 17, 128, 129, 192, 193)
+    E = len(counts)
+    banks, deq = [], []
+    for _ in range(2):
+        w = (torch.randn((E, N, K), generator=gen, device=DEV) * 0.1).to(dtype)
+        wq, s, b = jq.quantize(w, gs, bits)
+        banks.append(jq.ExpertBank(wq, s, b, bits, gs))
+        deq.append(jq.dequantize(wq, s, b, gs, bits, dtype=torch.float32).to(dtype).double())
+    idx = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)]).to(DEV)
+    idx = idx[torch.randperm(idx.numel(), generator=gen, device=DEV)].contiguous()
+    P = idx.numel()
+    x = torch.randn((P, K), generator=gen, device=DEV).to(dtype)
+    wts = torch.rand((P,), generator=gen, device=DEV)
+    lim = 1.5
+    sp = moe.SortedPairs(idx, E, tile_m=_lib.MOE_GEMM_TILE_M)
+    xs = moe._gather_rows(x, sp, 1)
+    h = torch.full((P + 1, N + 8), 7.0, dtype=dtype, device=DEV)
+    g, u = banks
+    dt = _lib.dtype_id(dtype)
+    _lib.check(lib.jq_moe_gate_up_swiglu(
+        xs.data_ptr(), dt, P, xs.stride(0), sp.offsets.data_ptr(), sp.tile_expert.data_ptr(), sp.tile_row0.data_ptr(),
+        sp.num_tiles.data_ptr(), sp.max_tiles, sp.tile_m, g.codes_tab.data_ptr(), g.scales_tab.data_ptr(),
+        g.biases_tab.data_ptr(), u.codes_tab.data_ptr(), u.scales_tab.data_ptr(), u.biases_tab.data_ptr(), dt, N, K, bits, gs,
+        wts.data_ptr(), sp.order.data_ptr(), lim, h.data_ptr(), h.stride(0), _lib.stream_ptr(torch.device(DEV))))
+    order = sp.order[:P].long()
+    e = idx[order].long()
+    xd = x[order].double()
+    gv = torch.einsum("pk,pnk->pn", xd, deq[0][e]).clamp(max=lim)
+    uv = torch.einsum("pk,pnk->pn", xd, deq[1][e]).clamp(-lim, lim)
+    ref = gv / (1 + torch.exp(-gv)) * uv * wts[order].double()[:, None]
+    got = h[:P, :N].double()
+    ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert torch.all((got - ref).abs() <= ulp * ref.abs() + 1e-3 * ref.abs().max())
+    assert bool((h[:P, N:] == 7.0).all()) and bool((h[P:] == 7.0).all())
+    _lib.check(lib.jq_device_status())

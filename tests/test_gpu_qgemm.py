@@ -148,3 +148,48 @@ def test_qgemm_split_k_over_a_cluster(bits, M, N, K, gs):
     y2 = jq.quantized_matmul(x, wq, s, b, group_size=gs, bits=bits)
     assert torch.equal(y, y2)                                  # the partial sums are added in rank order
     _lib.check(_lib.load().jq_device_status())
+
+
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
+@pytest.mark.parametrize("bits", (2, 3, 4, 5, 6, 8))
+@pytest.mark.parametrize("M,N,K,gs,scale", (
+    (17, 129, 128, 64, 0.02),      # two k-blocks: two of the four dequantizer groups stay idle; two groups per row
+    (33, 257, 384, 64, 0.02),      # six groups per row: two 4-byte sidecar copies per chunk, the last one half
+    (256, 128, 384, 128, 0.02),    # three groups per row: sidecars not staged; exactly one full row tile
+    (257, 100, 640, 64, 0.02),     # one row past a tile, ten groups per row
+    (70, 300, 2048, 128, 0.02),    # split K, one 4-byte copy per chunk
+    (100, 300, 1152, 64, 4.0),     # scales above the limit of the fast expansion: the general form
+    (90, 130, 256, 64, 200.0),
+))
+def test_qgemm_expansion_and_sidecar_forms(M, N, K, gs, scale, bits, dtype):
+    """Every way scales reach the dequantizers and both register expansions, at the edges of the k-block rotation."""
+    rng = np.random.default_rng(bits + M)
+    w = torch.from_numpy((rng.standard_normal((N, K)) * scale).astype(np.float32)).to(DEV).to(dtype)
+    x = torch.from_numpy(rng.standard_normal((M, K)).astype(np.float32)).to(DEV).to(dtype)
+    wq, s, b = jq.quantize(w, gs, bits)
+    y = jq.quantized_matmul(x, wq, s, b, group_size=gs, bits=bits)
+    check(y, x, wq, s, b, bits, gs, dtype)
+    _lib.check(_lib.load().jq_device_status())
+
+
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
+@pytest.mark.parametrize("bits", (2, 3, 4, 5, 6, 8))
+def test_qgemm_weight_operand_is_rounded_once(bits, dtype):
+    """x = identity returns the weight operand itself: rn(q * scale + bias), the dequantizer's values, bit for bit --
+    over scales from the subnormals of the activation type to above the limit of the fast expansion.  (8-bit codes of
+    large bfloat16 scales go through float32 and may round twice: one step.)"""
+    K, N, gs = 256, 192, 64
+    rng = np.random.default_rng(bits)
+    mag = np.exp2(rng.uniform(-12 if dtype == torch.float16 else -100, 6, size=(N, K // gs, 1)))
+    w = torch.from_numpy((rng.standard_normal((N, K // gs, gs)) * mag).astype(np.float32).reshape(N, K)).to(DEV).to(dtype)
+    wq, s, b = jq.quantize(w, gs, bits)
+    y = jq.quantized_matmul(torch.eye(K, dtype=dtype, device=DEV), wq, s, b, group_size=gs, bits=bits)
+    ref = jq.dequantize(wq, s, b, gs, bits, dtype=torch.float32).to(dtype).T
+    # -0 and +0 meet in the sum; a product with a subnormal weight is exact in the float32 accumulator
+    if bits == 8 and dtype == torch.bfloat16:
+        assert torch.all((y.float() - ref.float()).abs() <= ref.float().abs() * 2.0 ** -7 + 1e-38)
+    else:
+        exact = jq.dequantize(wq, s, b, gs, bits, dtype=torch.float32).T.double()
+        # the dequantizer rounds to float32 and then to 16 bits, the operand once: either neighbour of a tie
+        ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+        assert torch.all((y.double() - exact).abs() <= exact.abs() * ulp * (1 + 1e-4) + 6.1e-8 * (dtype == torch.float16))
