@@ -291,14 +291,30 @@ moe_sort_place_kernel(const int32_t* __restrict__ idx, int n, int E, int base, i
     }
 }
 
-// dst[p, :] = src[order[p] / div, :] for p < *count (16-byte vectors; cols*2 % 16 == 0)
-__global__ void gather_rows_kernel(const uint4* __restrict__ src, int64_t src_ld_vec, const int32_t* __restrict__ order,
+// dst[p, :] = src[order[p] / div, :] for p < *count (16-byte vectors; cols*2 % 16 == 0).  Bound: the write of the
+// copied rows.  A CTA copies one row at a time with up to four vectors per thread in flight, and the grid has a CTA
+// per row up to 32 per SM: a row is one dependent pair of loads (order, then the row), so what hides that latency is
+// the number of rows in flight.
+__global__ void __launch_bounds__(128)
+gather_rows_kernel(const uint4* __restrict__ src, int64_t src_ld_vec, const int32_t* __restrict__ order,
                                    const int32_t* __restrict__ count, int div, uint4* __restrict__ dst,
                                    int64_t dst_ld_vec, int cols_vec, int max_rows) {
     const int n = min(*count, max_rows);
     for (int p = blockIdx.x; p < n; p += gridDim.x) {
         const int64_t s = order[p] / div;
-        for (int c = threadIdx.x; c < cols_vec; c += blockDim.x) dst[p * dst_ld_vec + c] = __ldg(src + s * src_ld_vec + c);
+        const uint4* sp = src + s * src_ld_vec;
+        uint4* dp = dst + p * dst_ld_vec;
+        int c = threadIdx.x;
+        for (; c + 3 * 128 < cols_vec; c += 4 * 128) {
+            const uint4 v0 = __ldg(sp + c), v1 = __ldg(sp + c + 128), v2 = __ldg(sp + c + 256), v3 = __ldg(sp + c + 384);
+            dp[c] = v0; dp[c + 128] = v1; dp[c + 256] = v2; dp[c + 384] = v3;
+        }
+        if (c + 128 < cols_vec) {
+            const uint4 v0 = __ldg(sp + c), v1 = __ldg(sp + c + 128);
+            dp[c] = v0; dp[c + 128] = v1;
+            c += 256;
+        }
+        if (c < cols_vec) dp[c] = __ldg(sp + c);
     }
 }
 
@@ -368,14 +384,24 @@ __global__ void combine_kernel(const AT* __restrict__ y, int64_t ldy, const int3
                 float acc[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-                for (int j = 0; j < k; ++j) {
-                    const int p = inv ? inv[t * k + j] : t * k + j;
-                    if (p < 0) continue;
-                    const float wj = w ? w[t * k + j] : 1.0f;
-                    const uint4 q = __ldg(reinterpret_cast<const uint4*>(y + (int64_t)p * ldy + c));
-                    const AT* ya = reinterpret_cast<const AT*>(&q);
+                // eight slots at a time: their row numbers first, then all their vectors, so that the loads of a
+                // batch are in flight together (one after the other they are a chain of 2 k dependent loads)
+                for (int j0 = 0; j0 < k; j0 += 8) {
+                    int p[8];
+                    uint4 q[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i] = fmaf(wj, Elt<AT>::to_f32(ya[i]), acc[i]);
+                    for (int j = 0; j < 8; ++j) p[j] = j0 + j < k ? (inv ? inv[t * k + j0 + j] : t * k + j0 + j) : -1;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (p[j] >= 0) q[j] = __ldg(reinterpret_cast<const uint4*>(y + (int64_t)p[j] * ldy + c));
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (p[j] < 0) continue;
+                        const float wj = w ? w[t * k + j0 + j] : 1.0f;
+                        const AT* ya = reinterpret_cast<const AT*>(&q[j]);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[i] = fmaf(wj, Elt<AT>::to_f32(ya[i]), acc[i]);
+                    }
                 }
                 if (shared) {
                     const uint4 q = __ldg(reinterpret_cast<const uint4*>(shared + (int64_t)t * ld_shared + c));
@@ -708,15 +734,16 @@ route_cluster_kernel(const AT* __restrict__ x, const AT* __restrict__ wr, int H,
 // Router for many tokens (prefill): the logits come from a GEMM; one warp per token turns its row of logits
 // (f32, or the activation type) into the softmax over the experts in f32, the k largest scores (ties to the
 // lower id) and w = p / (sum p + 1e-20) * scale -- route_kernel's selection, one launch instead of the five or
-// six of an eager softmax / top-k / normalise chain.  E <= 1024: a lane holds up to 32 logits in registers.
-template <typename LT>
+// six of an eager softmax / top-k / normalise chain.  E <= 1024: a lane holds PER >= E / 32 logits in registers, and
+// PER is the smallest of 2, 4, 8, 16, 32 that covers E: every step of the k selections walks all PER of them, which
+// for 128 experts was eight times the needed instructions with a fixed 32.
+template <typename LT, int PER>
 __global__ void __launch_bounds__(256)
 topk_rows_kernel(const LT* __restrict__ logits, int64_t ld, int T, int E, int k, int renorm, float scale,
                  int32_t* __restrict__ idx_out, float* __restrict__ w_out) {
     const int lane = threadIdx.x & 31;
     const int t = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (t >= T) return;
-    constexpr int PER = ROUTE_MAX_E / 32;
     float p[PER];
     float mx = -INFINITY;
 #pragma unroll
@@ -896,14 +923,22 @@ int jq_moe_topk(const void* logits, int logits_dtype, int64_t ld, int64_t T, int
     JQ_REQUIRE(logits && idx_out && w_out, JQ_EINVAL, "null pointer");
     const unsigned blocks = (unsigned)((T * 32 + 255) / 256);
     cudaStream_t st = (cudaStream_t)stream;
-    if (logits_dtype == JQ_F32)
-        topk_rows_kernel<float><<<blocks, 256, 0, st>>>((const float*)logits, ld, (int)T, num_experts, k, renorm, scale, idx_out, w_out);
-    else if (logits_dtype == JQ_BF16)
-        topk_rows_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)logits, ld, (int)T, num_experts, k, renorm,
-                                                               scale, idx_out, w_out);
-    else if (logits_dtype == JQ_F16)
-        topk_rows_kernel<__half><<<blocks, 256, 0, st>>>((const __half*)logits, ld, (int)T, num_experts, k, renorm, scale, idx_out,
-                                                        w_out);
+#define JQ_TOPK(T_, P)                                                                                               \
+    topk_rows_kernel<T_, P><<<blocks, 256, 0, st>>>((const T_*)logits, ld, (int)T, num_experts, k, renorm, scale, idx_out, \
+                                                    w_out)
+#define JQ_TOPK_E(T_)                                                                                                \
+    {                                                                                                                \
+        if (num_experts <= 64) JQ_TOPK(T_, 2);                                                                       \
+        else if (num_experts <= 128) JQ_TOPK(T_, 4);                                                                 \
+        else if (num_experts <= 256) JQ_TOPK(T_, 8);                                                                 \
+        else if (num_experts <= 512) JQ_TOPK(T_, 16);                                                                \
+        else JQ_TOPK(T_, 32);                                                                                        \
+    }
+    if (logits_dtype == JQ_F32) JQ_TOPK_E(float)
+    else if (logits_dtype == JQ_BF16) JQ_TOPK_E(__nv_bfloat16)
+    else if (logits_dtype == JQ_F16) JQ_TOPK_E(__half)
+#undef JQ_TOPK_E
+#undef JQ_TOPK
     else
         return fail(JQ_EINVAL, "logits must be f32, f16 or bf16");
     return check_launch("moe_topk");
@@ -979,7 +1014,7 @@ int jq_gather_rows(const void* src, int64_t src_ld, const int32_t* order, const 
     JQ_REQUIRE(src && dst && order && count, JQ_EINVAL, "null pointer");
     JQ_REQUIRE(cols % 8 == 0 && src_ld % 8 == 0 && dst_ld % 8 == 0 && aligned(src, 16) && aligned(dst, 16), JQ_EINVAL,
                "gather_rows needs 16-byte aligned rows");
-    const int blocks = (int)(max_rows < 4 * 148 ? max_rows : 4 * 148);
+    const int blocks = (int)(max_rows < 32 * 148 ? max_rows : 32 * 148);
     gather_rows_kernel<<<blocks, 128, 0, (cudaStream_t)stream>>>((const uint4*)src, src_ld / 8, order, count, div,
                                                                   (uint4*)dst, dst_ld / 8, (int)(cols / 8), (int)max_rows);
     return check_launch("gather_rows");

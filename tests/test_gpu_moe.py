@@ -749,3 +749,43 @@ def test_gate_up_swiglu_in_one_launch(bits, K, N, gs, dtype):
     assert torch.all((got - ref).abs() <= ulp * ref.abs() + 1e-3 * ref.abs().max())
     assert bool((h[:P, N:] == 7.0).all()) and bool((h[P:] == 7.0).all())
     _lib.check(lib.jq_device_status())
+
+
+@pytest.mark.parametrize("dtype", (torch.float32, torch.bfloat16))
+@pytest.mark.parametrize("E", (8, 64, 65, 128, 129, 256, 257, 512, 513, 1024))
+def test_topk_over_every_register_count(E, dtype):
+    """jq_moe_topk holds 2, 4, 8, 16 or 32 logits per lane: ids exact (ties to the lower id), weights of the float32
+    softmax within 1e-5 relative (__expf and the order of the sum)."""
+    from jangq_b200.moe import route_softmax_topk
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(E)
+    T, k = 37, min(10, E)
+    logits = torch.randn((T, E), generator=gen, device=DEV).to(dtype)
+    idx, w = route_softmax_topk(logits, k)
+    p = torch.softmax(logits.double(), -1)
+    order = torch.sort(-logits.double(), dim=-1, stable=True).indices[:, :k]      # equal logits: ascending id
+    assert torch.equal(idx.long(), order)
+    ref = torch.gather(p, 1, order)
+    ref = ref / ref.sum(-1, keepdim=True)
+    assert torch.all((w.double() - ref).abs() <= 1e-5 * ref)
+
+
+@pytest.mark.parametrize("k", (1, 7, 8, 9, 17))
+@pytest.mark.parametrize("D", (8, 264, 2048))
+def test_combine_batches_of_eight_slots(k, D):
+    """Slots are loaded eight at a time and added in slot order: the float32 sums of the plain loop, bit for bit."""
+    lib = _lib.load()
+    T = 5
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(k + D)
+    y = torch.randn((T * k, D), generator=gen, device=DEV).to(torch.bfloat16)
+    inv = torch.randperm(T * k, generator=gen, device=DEV).to(torch.int32)
+    inv[::5] = -1                                                                  # pairs of another rank
+    out = torch.empty((T, D), dtype=torch.float32, device=DEV)
+    _lib.check(lib.jq_moe_combine(y.data_ptr(), D, inv.data_ptr(), None, T, k, D, None, D, out.data_ptr(), _lib.JQ_BF16,
+                                  _lib.stream_ptr(torch.device(DEV))))
+    ref = torch.zeros((T, D), dtype=torch.float32, device=DEV)
+    for j in range(k):
+        p = inv.view(T, k)[:, j].long()
+        ref += torch.where((p >= 0)[:, None], y[p.clamp(min=0)].float(), torch.zeros((), device=DEV))
+    assert torch.equal(out, ref)
