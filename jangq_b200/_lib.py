@@ -5,6 +5,7 @@ an exception is raised.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import os
 import threading
@@ -149,19 +150,31 @@ def dtype_id(dt: torch.dtype) -> int:
         raise JangqError(JQ_EINVAL, f"unsupported dtype {dt}; use float32, float16 or bfloat16") from None
 
 
+# A small call is a few microseconds of kernel, so what Python does around it is what the caller waits for: the raw
+# stream handle instead of a Stream object, no device switch when the device is current already, integers instead of
+# torch.device objects in the checks.
 def stream_ptr(device=None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = None if device is None else torch.device(device).index if isinstance(device, str) else device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+_same_device = contextlib.nullcontext()
+
+
+def on_device(dev: torch.device):
+    """Context manager that makes `dev` (of a CUDA tensor, so CUDA is initialised) the current device."""
+    return _same_device if torch._C._cuda_getDevice() == dev.index else torch.cuda.device(dev)
 
 
 def require_cuda(*tensors: torch.Tensor) -> torch.device:
-    dev = None
+    first, index = None, -1
     for t in tensors:
         if t is None:
             continue
         if not t.is_cuda:
             raise JangqError(JQ_EINVAL, "jangq_b200 ops take CUDA tensors only (there is no CPU path)")
-        if dev is None:
-            dev = t.device
-        elif t.device != dev:
-            raise JangqError(JQ_EINVAL, f"tensors on different devices: {dev} vs {t.device}")
-    return dev
+        if first is None:
+            first, index = t, t.get_device()
+        elif t.get_device() != index:
+            raise JangqError(JQ_EINVAL, f"tensors on different devices: {first.device} vs {t.device}")
+    return None if first is None else first.device

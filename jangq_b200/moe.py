@@ -240,7 +240,7 @@ def gather_qmm(x: torch.Tensor, w, scales: torch.Tensor | None = None, biases: t
     else:
         raise JangqError(_lib.JQ_EINVAL, f"cannot match {x2.shape[0]} rows of x with {R} indices")
     x2 = x2.contiguous()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         if R < SORT_THRESHOLD or not bank.gemm_ok:
             return _gather_qgemv(x2, x_div, rhs, bank)
         sp = SortedPairs(rhs, bank.E)
@@ -260,7 +260,7 @@ def route_softmax_topk(logits: torch.Tensor, k: int, renorm: bool = True, scale:
         T, E = logits.shape
         idx = torch.empty((T, k), dtype=torch.int32, device=logits.device)
         wts = torch.empty((T, k), dtype=torch.float32, device=logits.device)
-        with torch.cuda.device(logits.device):
+        with _lib.on_device(logits.device):
             _lib.check(lib.jq_moe_topk(logits.data_ptr(), _lib.dtype_id(logits.dtype), logits.stride(0), T, E, k,
                                        1 if renorm else 0, float(scale), idx.data_ptr(), wts.data_ptr(),
                                        _lib.stream_ptr(logits.device)))
@@ -285,7 +285,7 @@ def route_from_hidden(x: torch.Tensor, router_w: torch.Tensor, k: int, renorm: b
     idx = torch.empty((T, k), dtype=torch.int32, device=dev)
     w = torch.empty((T, k), dtype=torch.float32, device=dev)
     cnt, ws = _route_workspace(dev, T, E)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_moe_route(x.data_ptr(), _lib.dtype_id(x.dtype), x.stride(0), T, H, router_w.data_ptr(), E, k,
                                     1 if renorm else 0, float(scale), idx.data_ptr(), w.data_ptr(), cnt.data_ptr(),
                                     ws.data_ptr(), _lib.stream_ptr(dev)))
@@ -308,7 +308,7 @@ def route_norm_from_hidden(x: torch.Tensor, res: torch.Tensor, router_w: torch.T
     idx = torch.empty((T, k), dtype=torch.int32, device=dev)
     w = torch.empty((T, k), dtype=torch.float32, device=dev)
     cnt, ws = _route_workspace(dev, T, E)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_moe_route_norm(x.data_ptr(), res.data_ptr(), _lib.dtype_id(x.dtype), T, H, float(eps),
                                          xo.data_ptr(), router_w.data_ptr(), E, k, 1 if renorm else 0, float(scale),
                                          idx.data_ptr(), w.data_ptr(), cnt.data_ptr(), ws.data_ptr(), _lib.stream_ptr(dev)))
@@ -345,7 +345,7 @@ def residual_rmsnorm(x: torch.Tensor, y: torch.Tensor, eps: float | None = None,
         eps = torch.finfo(x.dtype).eps
     out = torch.empty_like(x)
     yf = y.dtype == torch.float32
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_residual_rmsnorm(x.data_ptr(), None if yf else y.data_ptr(), y.data_ptr() if yf else None, k, T, H,
                                            float(eps), out.data_ptr(), _lib.dtype_id(x.dtype), _lib.stream_ptr(dev)))
     return out
@@ -408,7 +408,7 @@ def moe_layer(x: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, gate: ExpertB
     dt = _lib.dtype_id(x.dtype)
     st = _lib.stream_ptr(dev)
     I = gate.N
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         use_sorted = P >= SORT_THRESHOLD if few_token_path is None else not few_token_path
         if use_sorted and gate.gemm_ok and up.gemm_ok and down.gemm_ok:
             # the grouped kernels take up to 192 rows of an expert per tile, and as many MMA columns as there are rows

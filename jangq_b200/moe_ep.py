@@ -140,7 +140,7 @@ def dispatch_combine_slots(x: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, 
     out = torch.empty((T, y_back.shape[1]), dtype=torch.float32, device=dev)
     if x.is_cuda:
         lib = _lib.load()
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             _lib.check(lib.jq_moe_combine(y_back.data_ptr(), y_back.stride(0), slot_of_pair.data_ptr(), None, T, k,
                                           y_back.shape[1], None, y_back.shape[1], out.data_ptr(),
                                           _lib.dtype_id(x.dtype), _lib.stream_ptr(dev)))
@@ -168,7 +168,7 @@ def _dispatch_combine_slots_cuda(x, idx, w, num_experts, local_fn, C, group, wor
     slot_of_pair = torch.empty(max(T * k, 1), dtype=torch.int32, device=dev)
     scratch = torch.empty(world + 1, dtype=torch.int32, device=dev)           # counters, then the overflow word
     st = _lib.stream_ptr(dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_ep_pack_slots(x.data_ptr(), x.stride(0), idx32.data_ptr(), wf.data_ptr(), T, k, H, num_experts,
                                         world, C, send.data_ptr(), slot_of_pair.data_ptr(), scratch.data_ptr(),
                                         scratch[world:].data_ptr(), st))
@@ -287,7 +287,7 @@ def peer_combine_residual_rmsnorm(x: torch.Tensor, y: torch.Tensor, k: int, ex: 
     if eps is None:
         eps = torch.finfo(x.dtype).eps
     out = torch.empty_like(x)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_ep_combine_residual_rmsnorm(
             x.data_ptr(), y.data_ptr(), k, T, H, float(eps), out.data_ptr(), _lib.dtype_id(x.dtype), ex._ptr_array,
             0 if emul else ex.rank, ex.world, ex.tcap, ex.counters.data_ptr(), ex.world if emul else 0,

@@ -14,6 +14,7 @@ import torch
 
 from . import _lib
 from ._lib import JangqError
+from .gemm import qgemm
 
 ALLOWED_BITS = (2, 3, 4, 5, 6, 8)
 ALLOWED_GROUP_SIZES = (32, 64, 128)
@@ -32,13 +33,14 @@ def _check_triple(wq, scales, biases, bits, group_size):
         raise JangqError(_lib.JQ_EUNSUPPORTED, f"unsupported bits={bits}")
     if group_size not in ALLOWED_GROUP_SIZES:
         raise JangqError(_lib.JQ_EUNSUPPORTED, f"unsupported group_size={group_size}")
-    K = wq.shape[-1] * 32 // bits
-    if wq.shape[-1] * 32 % bits or K % group_size:
+    wshape, sshape = wq.shape, scales.shape
+    K = wshape[-1] * 32 // bits
+    if wshape[-1] * 32 % bits or K % group_size:
         raise JangqError(_lib.JQ_EINVAL, f"packed width {wq.shape[-1]} does not match bits={bits}, "
                                          f"group_size={group_size}")
-    if scales.shape != biases.shape or scales.dtype != biases.dtype:
+    if sshape != biases.shape or scales.dtype != biases.dtype:
         raise JangqError(_lib.JQ_EINVAL, "scales and biases must share shape and dtype")
-    if tuple(scales.shape) != tuple(wq.shape[:-1]) + (K // group_size,):
+    if len(sshape) != len(wshape) or sshape[-1] != K // group_size or sshape[:-1] != wshape[:-1]:
         raise JangqError(_lib.JQ_EINVAL, f"scales shape {tuple(scales.shape)} does not match codes "
                                          f"{tuple(wq.shape)} at bits={bits}, group_size={group_size}")
     return K
@@ -63,8 +65,9 @@ def quantize(w: torch.Tensor, group_size: int = 64, bits: int = 4, *, sidecar_dt
     K = w.shape[-1]
     if K == 0:
         raise JangqError(_lib.JQ_EINVAL, "affine quantization expects rows of at least one group")
+    matrix = w.dim() == 2
     lead = tuple(w.shape[:-1])
-    w2 = w.reshape(-1, K).contiguous()
+    w2 = (w if matrix else w.reshape(-1, K)).contiguous()
     rows = w2.shape[0]
     if mode in ("rtn", "rtn_ieee_div", "mse", "mse_exhaustive") and sidecar_dtype is None:
         sidecar_dtype = torch.float16
@@ -76,7 +79,7 @@ def quantize(w: torch.Tensor, group_size: int = 64, bits: int = 4, *, sidecar_dt
     G = K // group_size if group_size in ALLOWED_GROUP_SIZES else 0
     scales = torch.empty((rows, G), dtype=sdt, device=dev)
     biases = torch.empty((rows, G), dtype=sdt, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         if mode in ("affine", "affine_ieee_div"):
             flags = _lib.JQ_QUANT_F16_TINY_GUARD if f16_tiny_guard else 0
             if mode == "affine_ieee_div":
@@ -96,6 +99,8 @@ def quantize(w: torch.Tensor, group_size: int = 64, bits: int = 4, *, sidecar_dt
                                            biases.data_ptr(), _lib.stream_ptr(dev)))
         else:
             raise JangqError(_lib.JQ_EINVAL, f"unknown quantize mode {mode!r}")
+    if matrix:
+        return wq, scales, biases
     return wq.reshape(lead + (wq.shape[-1],)), scales.reshape(lead + (G,)), biases.reshape(lead + (G,))
 
 
@@ -111,7 +116,7 @@ def dequantize(wq: torch.Tensor, scales: torch.Tensor, biases: torch.Tensor, gro
         biases.reshape(-1, biases.shape[-1]).contiguous()
     rows = wq2.shape[0]
     out = torch.empty((rows, K), dtype=dtype or scales.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_dequantize(wq2.data_ptr(), s2.data_ptr(), b2.data_ptr(), _lib.dtype_id(s2.dtype), rows, K,
                                      bits, group_size, out.data_ptr(), _lib.dtype_id(out.dtype),
                                      _lib.stream_ptr(dev)))
@@ -146,7 +151,7 @@ def quantize_imatrix(w: torch.Tensor, importance, group_size: int = 64, bits: in
     s = torch.empty((rows, K // group_size), dtype=torch.float16, device=dev)
     b = torch.empty_like(s)
     impd = torch.from_numpy(imp).to(dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_quantize_imatrix(w2.data_ptr(), _lib.dtype_id(w2.dtype), impd.data_ptr(), rows, K, bits,
                                            group_size, iterations, wq.data_ptr(), s.data_ptr(), b.data_ptr(),
                                            _lib.stream_ptr(dev)))
@@ -182,7 +187,7 @@ def hadamard_rotate(x: torch.Tensor, signs: torch.Tensor | None = None, seed: in
         raise JangqError(_lib.JQ_EINVAL, f"signs must be float32 [{K}], got {signs.dtype} {tuple(signs.shape)}")
     x2 = x.reshape(-1, K).contiguous()
     out = torch.empty((x2.shape[0], K), dtype=dtype or x.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_hadamard_rotate(x2.data_ptr(), _lib.dtype_id(x2.dtype), K, x2.shape[0], K, signs.data_ptr(),
                                           out.data_ptr(), _lib.dtype_id(out.dtype), K, _lib.stream_ptr(dev)))
     return out.reshape(tuple(x.shape[:-1]) + (K,))
@@ -202,7 +207,7 @@ def embedding(ids: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases:
     wq, scales, biases = wq.contiguous(), scales.contiguous(), biases.contiguous()
     flat = ids.reshape(-1).to(torch.int32).contiguous()
     out = torch.empty((flat.numel(), K), dtype=dtype or scales.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_embedding(flat.data_ptr(), flat.numel(), wq.data_ptr(), scales.data_ptr(), biases.data_ptr(),
                                     _lib.dtype_id(scales.dtype), wq.shape[0], K, bits, group_size, out.data_ptr(),
                                     _lib.dtype_id(out.dtype), _lib.stream_ptr(dev)))
@@ -286,24 +291,24 @@ def quantized_matmul(x: torch.Tensor, w: torch.Tensor, scales: torch.Tensor, bia
     if w.dim() != 2:
         raise JangqError(_lib.JQ_EINVAL, f"weight must be 2-D [N, K*bits/32], got {tuple(w.shape)}")
     K = _check_triple(w, scales, biases, bits, group_size)
-    if x.shape[-1] != K:
+    xshape = x.shape
+    if xshape[-1] != K:
         raise JangqError(_lib.JQ_EINVAL, f"x has {x.shape[-1]} features, weight expects {K}")
     if x.dtype not in (torch.bfloat16, torch.float16):
         raise JangqError(_lib.JQ_EINVAL, f"activations must be bfloat16 or float16, got {x.dtype}")
-    lead = tuple(x.shape[:-1])
-    x2 = x.reshape(-1, K)
+    matrix = len(xshape) == 2
+    x2 = x if matrix else x.reshape(-1, K)
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
     M, N = x2.shape[0], w.shape[0]
     w, scales, biases = w.contiguous(), scales.contiguous(), biases.contiguous()
     out = torch.empty((M, N), dtype=x.dtype, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         if M <= _lib.QGEMV_MAX_M:
             if M > 0:
                 _qgemv(x2, w, scales, biases, K, bits, group_size, out,
                        _lib.JQ_GEMV_STATIC_WEIGHTS if static_weights else 0)
         elif K % 64 == 0 and (K * bits // 8) % 16 == 0:
-            from .gemm import qgemm
             qgemm(x2, w, scales, biases, K, bits, group_size, out)
         else:
             # row lengths the tensor-core kernel does not take (K not a multiple of 64, or packed
@@ -311,4 +316,4 @@ def quantized_matmul(x: torch.Tensor, w: torch.Tensor, scales: torch.Tensor, bia
             for m0 in range(0, M, _lib.QGEMV_MAX_M):
                 _qgemv(x2[m0:m0 + _lib.QGEMV_MAX_M], w, scales, biases, K, bits, group_size,
                        out[m0:m0 + _lib.QGEMV_MAX_M])
-    return out.reshape(lead + (N,))
+    return out if matrix else out.reshape(tuple(xshape[:-1]) + (N,))

@@ -89,7 +89,7 @@ def tq_quantize_weight(weight: torch.Tensor, bits: int = 2, seed: int = 42) -> d
     rows = w2.shape[0]
     packed = torch.empty((rows, words), dtype=torch.int32, device=dev)
     norms = torch.empty((rows,), dtype=torch.float16, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_tq_quantize(w_rot.data_ptr(), rows, K, bits, edges.data_ptr(), packed.data_ptr(),
                                       norms.data_ptr(), _lib.stream_ptr(dev)))
     return {"packed": packed.reshape(lead + (words,)), "norms": norms.reshape(lead)}
@@ -113,7 +113,7 @@ def tq_gather_matmul(x_rot: torch.Tensor, packed: torch.Tensor, norms: torch.Ten
         rhs = rhs_indices.reshape(-1).to(torch.int32).contiguous()
         pairs, rhs_ptr = rhs.numel(), rhs.data_ptr()
     out = torch.empty((pairs, N), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_tq_gather_matmul(x_rot.data_ptr(), x_rot.stride(0), x_div, rhs_ptr, pairs,
                                            ops._as_i32(packed).contiguous().data_ptr(), norms.contiguous().data_ptr(),
                                            codebook.data_ptr(), E, N, K, bits, out.data_ptr(), out.stride(0),
@@ -134,7 +134,7 @@ def tq_fused_gate_up_swiglu(x_rot: torch.Tensor, gate: "TurboQuantSwitchLinear",
     k = rhs_indices.shape[-1] if rhs_indices.dim() == 2 else 1
     rhs = rhs_indices.reshape(-1).to(torch.int32).contiguous()
     out = torch.empty((rhs.numel(), gate.out_features), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.jq_tq_fused_gate_up_swiglu(x_rot.data_ptr(), x_rot.stride(0), k, rhs.data_ptr(), rhs.numel(),
                                                   gate.packed.data_ptr(), gate.norms.data_ptr(), up.packed.data_ptr(),
                                                   up.norms.data_ptr(), gate.codebook.data_ptr(), gate.num_experts,
