@@ -525,11 +525,17 @@ int qgemv_dispatch_items(const void* x, int x_dtype, int64_t M, int64_t ldx, con
     }
     if (live.count == 0) return JQ_OK;
     const int kern = gemv_kernel_choice();
-    for (int64_t m0 = 0; m0 < M; m0 += 8) {
+    // More than eight rows: one launch of the small-batch tensor-memory kernel instead of two of eight rows (16 rows,
+    // 14336x4096 4-bit 26 us against 52).  It also takes 8-bit codes from six rows on, where the limbs of the other
+    // tensor-memory kernel outgrow 16 columns (8 rows: 14336x4096 23 us against 30, 4096x4096 11.8 against 14.7; five
+    // rows tie).  At eight rows of narrower codes it ties or loses (4-bit 24.5 against 23.7 us, 2-bit 4096x4096 11.5
+    // against 9.6).
+    int64_t step = fast && kern == 0 && (M > 8 || (bits == 8 && M > 5)) ? 16 : 8;
+    for (int64_t m0 = 0; m0 < M; m0 += step) {
         GemvArgs a = {};
         a.x = (const char*)x + m0 * ldx * dtype_size(x_dtype);
         a.K = K; a.ldx = ldx;
-        a.M = (int)((M - m0) < 8 ? (M - m0) : 8);
+        a.M = (int)((M - m0) < step ? (M - m0) : step);
         a.G = (int)(K / gs);
         a.pdl = (flags & JQ_GEMV_STATIC_WEIGHTS) ? 1 : 0;
         a.x_div = 1; a.ksplit = 1;
@@ -544,6 +550,13 @@ int qgemv_dispatch_items(const void* x, int x_dtype, int64_t M, int64_t ldx, con
         a.N = bt.N[0]; a.ldy = bt.ldy[0];
         bool launched = false;
         int rc = JQ_OK;
+        if (step == 16) {
+            rc = launch_ts_kernel(a, bt, x_dtype, bits, gs, st, &launched);
+            if (rc != JQ_OK) return rc;
+            if (launched) continue;
+            step = 8;
+            a.M = (int)((M - m0) < step ? (M - m0) : step);
+        }
         // Measured choice on B200 (CUDA events, overlapped launches, working set >> L2):
         //   2-, 4- and 8-bit, M <= 2: persistent integer warp-MMA kernel (22016x4096 2-bit: 12.0 us against
         //          16.2 us for the per-tile integer kernel; 14336x4096 4-bit: 10.2 us and 32000x4096 8-bit:

@@ -36,7 +36,8 @@ struct GemvArgs {
     int64_t norm_ldy;
     int norm_k;
     float norm_eps;
-    int* status;  // device status word, set to 1 when a bounded wait ran out (tensor-memory kernel)
+    int* status;  // device status word, set to 1 when a bounded wait ran out (tensor-memory kernels)
+    int gs_shift; // small-batch tensor-memory kernel: log2 of the 64-code k-blocks per group
 };
 
 // Matrices of one fused launch: they share the activations (x, ldx), K, the bit width and the group
@@ -165,6 +166,10 @@ int launch_pint_kernel(const GemvArgs& a, const GemvBatch& bt, int act_dtype, in
 // tensor-memory kernel (jq_qgemv_tc.cu), dense mat-vecs only; *launched stays false when the shape does
 // not fit it and the caller should use the warp-MMA kernel instead
 int launch_tc_kernel(const GemvArgs& a, const GemvBatch& bt, int act_dtype, int bits, int gs, cudaStream_t st,
+                     bool* launched);
+
+// small-batch kernel (jq_qgemv_ts.cu): up to 16 activation rows in one launch, any width but 5; same convention
+int launch_ts_kernel(const GemvArgs& a, const GemvBatch& bt, int act_dtype, int bits, int gs, cudaStream_t st,
                      bool* launched);
 
 }  // namespace jq

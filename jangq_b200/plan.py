@@ -61,7 +61,7 @@ class GemvPlan:
         for g in self.groups:
             if any(self.x[i] is not self.x[g[0]] for i in g):
                 raise _lib.JangqError(_lib.JQ_EINVAL, "the linears of a group must read the same input buffer")
-        self.launches_per_run = sum(self._launches_of(g) for g in self.groups) * ((m + 7) // 8)
+        self.launches_per_run = sum(self._launches_of(g) * self._row_steps(g, m) for g in self.groups)
         # persistent: segments = ("program", StreamProgram) or ("groups", [group, ...]) in execution order
         self.persistent = bool(persistent) and m == 1
         self._segments = None
@@ -90,6 +90,12 @@ class GemvPlan:
         n, k = lin.out_features, lin.in_features
         e = lin.scales.element_size()
         return n * k * lin.bits // 8 + n * (k // lin.group_size) * 2 * e + m * k * 2 + m * n * 2
+
+    def _row_steps(self, group, m: int) -> int:
+        """Launches per matrix run for m rows: one up to 8 rows, and up to 16 where the small-batch kernel fits."""
+        lin = self.linears[group[0]]
+        fits = lin.bits != 5 and lin.group_size in (64, 128) and (lin.in_features // lin.group_size) % 4 == 0
+        return 1 if m <= 8 or fits else (m + 7) // 8
 
     def _launches_of(self, group) -> int:
         """Kernel launches of one group: runs of up to 4 consecutive members with equal (K, bits, group size)."""

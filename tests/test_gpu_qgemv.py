@@ -417,3 +417,24 @@ def test_row_formed_in_the_launch_validation():
     d[0].x = x.data_ptr()
     assert call(x.data_ptr(), ldy=K + 8) == _lib.JQ_EUNSUPPORTED
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
+@pytest.mark.parametrize("bits", (2, 3, 4, 6, 8))
+@pytest.mark.parametrize("M,N,K,gs", ((6, 129, 256, 64), (8, 1, 512, 128), (9, 127, 1024, 64), (16, 300, 2304, 64),
+                                      (13, 4096, 2048, 128), (16, 40000, 256, 64)))
+def test_small_batch_kernel(M, N, K, gs, bits, dtype):
+    """More than eight rows (six for 8-bit codes) in one launch: one to 36 k-blocks, K split over 1 to 8 CTAs, ragged row
+    tiles.  Codes are exact and scales unrounded, so against float64 only the float32 sums (1e-5 of the largest output)
+    and the output's rounding remain."""
+    gen = torch.Generator(device="cuda:0")
+    gen.manual_seed(M * 7 + bits)
+    w = (torch.randn((N, K), generator=gen, device="cuda:0") * 0.02).to(dtype)
+    x = torch.randn((M, K), generator=gen, device="cuda:0").to(dtype)
+    wq, s, b = jq.quantize(w, gs, bits)
+    y = jq.quantized_matmul(x, wq, s, b, group_size=gs, bits=bits)
+    ref = x.double() @ jq.dequantize(wq, s, b, gs, bits, dtype=torch.float32).double().T
+    ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert torch.all((y.double() - ref).abs() <= ulp * ref.abs() + 1e-5 * ref.abs().max())
+    assert torch.equal(y, jq.quantized_matmul(x, wq, s, b, group_size=gs, bits=bits))      # rank order: reproducible
+    _lib.check(_lib.load().jq_device_status())
