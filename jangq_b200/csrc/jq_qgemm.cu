@@ -427,7 +427,8 @@ template <int BITS> struct PersCfg {
     static constexpr int NBAR = 2 * RA + 2 * CD + 2 * ND;
     static constexpr int SIDE_OFF = RA * X_STAGE + CD * C_STAGE;
     static constexpr int SW_OFF = SIDE_OFF + CD * SIDE_SLOT;             // float[32][128]: gate/up exchange
-    static constexpr int BAR_OFF = SW_OFF + 32 * 128 * 4;
+    static constexpr int WT_OFF = SW_OFF + 32 * 128 * 4;                 // float[192]: routing weights of the tile's rows
+    static constexpr int BAR_OFF = WT_OFF + TNMAX * 4;
     static constexpr size_t SMEM = 1024 + BAR_OFF + NBAR * 8 + 16;
 };
 
@@ -580,6 +581,13 @@ qgemm_pers_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
         for (int tile = first; tile < total && ok; tile += step) {
             const PersTile t = take(tile);
             if (t.rows <= 0) continue;
+            if constexpr (GU) {
+                // the rows' routing weights while the MMAs run: fetched in the loop below they are two dependent loads per
+                // step and made the epilogue as long as the k-loop (2048 tokens, 128 experts: 161 us for the launch).
+                // The last barrier of the previous tile has released the buffer.
+                float* wt = reinterpret_cast<float*>(smem + C::WT_OFF);
+                for (int q = r; q < t.rows; q += 128) wt[q] = a.wts ? a.wts[a.order[t.m0 + q]] : 1.0f;
+            }
             ok = __all_sync(0xFFFFFFFFu, ts_wait(accfull + d, dph));
             if constexpr (GU) {      // the four warps meet in barriers below: they go on or leave together
                 int all;
@@ -611,8 +619,7 @@ qgemm_pers_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
                         const float4 g4 = *reinterpret_cast<const float4*>(sw + tok * 128 + nl);
                         const float4 u4 = *reinterpret_cast<const float4*>(sw + tok * 128 + 64 + nl);
                         const int64_t row = t.m0 + c0 + tok;
-                        const float wt = a.wts ? a.wts[a.order[row]] : 1.0f;
-                        store_swiglu<AT>(a, g4, u4, wt, row, t.n0 + nl);
+                        store_swiglu<AT>(a, g4, u4, reinterpret_cast<const float*>(smem + C::WT_OFF)[c0 + tok], row, t.n0 + nl);
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                 } else {
