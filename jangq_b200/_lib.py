@@ -154,7 +154,9 @@ def dtype_id(dt: torch.dtype) -> int:
 # stream handle instead of a Stream object, no device switch when the device is current already, integers instead of
 # torch.device objects in the checks.
 def stream_ptr(device=None) -> int:
-    index = None if device is None else torch.device(device).index if isinstance(device, str) else device.index
+    if device is not None and not isinstance(device, torch.device):
+        device = torch.device("cuda", device) if isinstance(device, int) else torch.device(device)
+    index = None if device is None else device.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 

@@ -53,11 +53,9 @@ class JANGLinear(nn.Module):
         return m
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        buf = self._buffers           # one dictionary instead of four attribute lookups through nn.Module
-        y = ops.quantized_matmul(x, buf["weight"], buf["scales"], buf["biases"], transpose=True,
+        y = ops.quantized_matmul(x, self.weight, self.scales, self.biases, transpose=True,
                                  group_size=self.group_size, bits=self.bits, static_weights=self.static_weights)
-        bias = buf["bias"]
-        return y if bias is None else y + bias
+        return y if self.bias is None else y + self.bias
 
     def extra_repr(self) -> str:
         return f"in={self.in_features}, out={self.out_features}, bits={self.bits}, group_size={self.group_size}"
