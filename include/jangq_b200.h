@@ -214,7 +214,10 @@ int jq_qgemm(const void* x, int x_dtype, int64_t M, int64_t ldx, const uint32_t*
  * Expert weights are addressed through DEVICE arrays of per-expert device pointers
  * (codes_tab/scales_tab/biases_tab, num_experts entries) so that every expert may have its
  * own bit width: bits_tab (device int32[num_experts], or NULL when all experts share `bits`)
- * makes a launch skip the experts whose width is not `bits`; call once per distinct width. */
+ * makes a launch skip the experts whose width is not `bits`; call once per distinct width.
+ * The pointers in the tables cannot be checked on the host.  Codes start on 16-byte boundaries.  Scales and biases do
+ * for jq_gather_qgemv*; the grouped GEMMs take them at any element, each expert its own way (staged 8 or 4 bytes at a
+ * time where they are aligned for it). */
 #define JQ_MOE_TILE_M 128
 
 /* Upper bound of the number of row tiles jq_moe_sort can emit (sizes tile_expert/tile_row0). */

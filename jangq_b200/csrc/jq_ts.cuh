@@ -352,16 +352,18 @@ __device__ __forceinline__ bool load_codes(const uint32_t* codes, int64_t n0, in
             const int col = CPR == 4 ? (l & 3) : (l + 64 * j) % CPR;
             if (col * 16 < rem) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dj), "l"(s) : "memory");
         }
-        if (side.mode != 0 && ((st0 + st) * CKB) % 4 == 0) {
-            const uint32_t sd = smem_u32(sSide) + (uint32_t)(slot * SIDE_SLOT + l * 8);
+        if (((st0 + st) * CKB) % 4 == 0) {             // a chunk has its slot whether it is staged or not: the mode may
+            if (side.mode != 0) {                      // change from tile to tile, and the dequantizers count every chunk
+                const uint32_t sd = smem_u32(sSide) + (uint32_t)(slot * SIDE_SLOT + l * 8);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {                                  // scales of both rows, then biases
-                const uint32_t di = sd + (uint32_t)(i * 64 * 8);
-                if (side.mode == 1) {
-                    cp_async_small<8>(di, sp[i] + soffb);
-                } else {
-                    cp_async_small<4>(di, sp[i] + soffb);
-                    if (side.mode == 2 && soffb + 4 < (int)side.G * 2) cp_async_small<4>(di + 4, sp[i] + soffb + 4);
+                for (int i = 0; i < 4; ++i) {                              // scales of both rows, then biases
+                    const uint32_t di = sd + (uint32_t)(i * 64 * 8);
+                    if (side.mode == 1) {
+                        cp_async_small<8>(di, sp[i] + soffb);
+                    } else {
+                        cp_async_small<4>(di, sp[i] + soffb);
+                        if (side.mode == 2 && soffb + 4 < (int)side.G * 2) cp_async_small<4>(di + 4, sp[i] + soffb + 4);
+                    }
                 }
             }
             soffb += chunk_bytes;

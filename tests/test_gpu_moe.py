@@ -789,3 +789,65 @@ def test_combine_batches_of_eight_slots(k, D):
         p = inv.view(T, k)[:, j].long()
         ref += torch.where((p >= 0)[:, None], y[p.clamp(min=0)].float(), torch.zeros((), device=DEV))
     assert torch.equal(out, ref)
+
+
+def grouped(x, sp, bank, tabs=None):
+    """jq_moe_gemm_tiled over every width of `bank`; tabs replaces its (scales, biases) pointer tables."""
+    lib = _lib.load()
+    dt = _lib.dtype_id(x.dtype)
+    stab, btab = tabs or (bank.scales_tab, bank.biases_tab)
+    y = torch.full((x.shape[0] + 1, bank.N + 8), 7.0, dtype=x.dtype, device=DEV)
+    for bits in bank.distinct_bits:
+        _lib.check(lib.jq_moe_gemm_tiled(
+            x.data_ptr(), dt, sp.n, x.stride(0), sp.offsets.data_ptr(), sp.tile_expert.data_ptr(), sp.tile_row0.data_ptr(),
+            sp.num_tiles.data_ptr(), sp.max_tiles, sp.tile_m, bank.codes_tab.data_ptr(), stab.data_ptr(), btab.data_ptr(),
+            bank.bits_tab.data_ptr() if bank.bits_tab is not None else None, dt, bank.N, bank.K, bits, bank.group_size,
+            y.data_ptr(), y.stride(0), _lib.stream_ptr()))
+    assert bool((y[:sp.n, bank.N:] == 7.0).all()) and bool((y[sp.n:] == 7.0).all())
+    return y[:sp.n, :bank.N]
+
+
+def gate_up(x, sp, gate, up, tabs=None):
+    """jq_moe_gate_up_swiglu without clamp and routing weights; tabs replaces the four sidecar pointer tables."""
+    lib = _lib.load()
+    dt = _lib.dtype_id(x.dtype)
+    gs_, gb, us, ub = tabs or (gate.scales_tab, gate.biases_tab, up.scales_tab, up.biases_tab)
+    h = torch.full((x.shape[0] + 1, gate.N + 8), 7.0, dtype=x.dtype, device=DEV)
+    _lib.check(lib.jq_moe_gate_up_swiglu(
+        x.data_ptr(), dt, sp.n, x.stride(0), sp.offsets.data_ptr(), sp.tile_expert.data_ptr(), sp.tile_row0.data_ptr(),
+        sp.num_tiles.data_ptr(), sp.max_tiles, sp.tile_m, gate.codes_tab.data_ptr(), gs_.data_ptr(), gb.data_ptr(),
+        up.codes_tab.data_ptr(), us.data_ptr(), ub.data_ptr(), dt, gate.N, gate.K, gate.distinct_bits[0], gate.group_size,
+        None, None, 0.0, h.data_ptr(), h.stride(0), _lib.stream_ptr()))
+    assert bool((h[:sp.n, gate.N:] == 7.0).all()) and bool((h[sp.n:] == 7.0).all())
+    return h[:sp.n, :gate.N]
+
+
+@pytest.mark.parametrize("bits,K,gs", ((4, 320, 64), (2, 384, 64), (3, 512, 64), (8, 512, 64), (6, 768, 128)))
+def test_grouped_gemm_experts_of_mixed_sidecar_alignment(bits, K, gs):
+    """Experts whose scales and biases start on 16-, 8-, 4- and 2-byte boundaries in one tile list, several tiles per CTA:
+    how a tile's scales reach the dequantizers changes from tile to tile, the products do not (bit for bit)."""
+    E, N = 48, 1152
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(K + bits)
+    counts = torch.randint(1, 40, (E,), generator=gen, device=DEV)
+    idx = torch.repeat_interleave(torch.arange(E, device=DEV, dtype=torch.int32), counts)
+    banks, tabs, keep = [], [], []
+    for _ in range(2):
+        w = (torch.randn((E, N, K), generator=gen, device=DEV) * 0.1).bfloat16()
+        bank = jq.ExpertBank(*jq.quantize(w, gs, bits), bits, gs)
+        banks.append(bank)
+        for side in (bank.scales, bank.biases):
+            ptrs = []
+            for e in range(E):
+                flat = torch.empty(side[e].numel() + 8, dtype=side.dtype, device=DEV)
+                part = flat[(0, 1, 4, 2, 1)[(e + len(tabs)) % 5]:][:side[e].numel()]
+                part.copy_(side[e].reshape(-1))
+                keep.append(flat)
+                ptrs.append(part.data_ptr())
+            tabs.append(torch.tensor(ptrs, dtype=torch.int64, device=DEV))
+    x = torch.randn((idx.numel(), K), generator=gen, device=DEV).bfloat16()
+    for tile_m in (128, 192):
+        sp = SortedPairs(idx, E, tile_m=tile_m)
+        assert torch.equal(grouped(x, sp, banks[0], tabs[:2]), grouped(x, sp, banks[0]))
+        assert torch.equal(gate_up(x, sp, *banks, tabs), gate_up(x, sp, *banks))
+    _lib.check(_lib.load().jq_device_status())
