@@ -295,14 +295,21 @@ __host__ __device__ inline int side_mode(const void* scales, const void* biases,
     return gs == 128 && G % 2 == 0 && at % 4 == 0 ? 3 : 0;
 }
 constexpr int SIDE_SLOT = 2 * 128 * 8;                    // bytes of a chunk: scales [128][4], then biases
+// base + row * pitch with a 64-bit product (rows of 2^31 bytes are taken, so 128 of them do not fit 32 bits), where it
+// stands: computed ahead, the addresses would take two registers each for the length of a loop
+__device__ __forceinline__ const uint8_t* row_at(const uint8_t* base, uint32_t row, uint32_t pitch) {
+    uint64_t p;
+    asm volatile("mad.wide.u32 %0, %1, %2, %3;" : "=l"(p) : "r"(row), "r"(pitch), "l"(base));
+    return reinterpret_cast<const uint8_t*>(p);
+}
 template <int N> __device__ __forceinline__ void cp_async_small(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(N) : "memory");
 }
 
 // The loader warps' loop: 64 lanes (l) copy nst stages of 128*WT rows, starting at stage st0 of the rows, into a ring
 // of CD stages; consecutive lanes take consecutive 16-byte chunks of a row, completion is counted on cfull (64
-// arrivals).  A lane's chunks keep their rows and columns from stage to stage, so their offsets are computed once: one
-// add and one copy per chunk are left in the loop (a warp alone on its scheduler issues an instruction every ~6 cycles;
+// arrivals).  A lane's chunks keep their rows and columns from stage to stage, so only one multiply-add and one copy per
+// chunk are left in the loop (a warp alone on its scheduler issues an instruction every ~6 cycles;
 // with the addresses computed per stage the loaders set the pace of the whole CTA).  (buf, phase) is the ring position,
 // (0, 1) at the start: the first pass finds every stage empty.  Returns false when a wait ran out; the caller waits for
 // the copies in flight.
@@ -318,16 +325,16 @@ __device__ __forceinline__ bool load_codes(const uint32_t* codes, int64_t n0, in
     const int last = (int)min((int64_t)((PAIR ? 64 : 128 * WT) - 1), N - 1 - n0);       // rows past N repeat the last one
     const uint8_t* src = reinterpret_cast<const uint8_t*>(codes) + n0 * (int64_t)rowbytes + (int64_t)st0 * RB;
     const int64_t second = PAIR ? reinterpret_cast<const uint8_t*>(codes2) - reinterpret_cast<const uint8_t*>(codes) : 0;
-    uint32_t soff[NCH];                                                     // < 2^31: 256 rows of less than 2^23 bytes
-    const uint32_t dst0 = smem_u32(sC);
-    uint32_t doff[CPR == 4 ? 1 : NCH];
+    uint32_t row[NCH];
 #pragma unroll
-    for (int j = 0; j < NCH; ++j) {
-        const int c = l + 64 * j, row = c / CPR, col = c - row * CPR;
-        soff[j] = (uint32_t)min(PAIR ? row & 63 : row, last) * rowbytes + (uint32_t)(col * 16);
-        // CPR == 4: the chunks of a lane are 16 rows apart and keep their swizzled column
-        if (CPR != 4 || j == 0) doff[CPR == 4 ? 0 : j] = (uint32_t)(row * RB + code_chunk<CPR>(col, row) * 16);
-    }
+    for (int j = 0; j < NCH; ++j) row[j] = (uint32_t)min(PAIR ? (l + 64 * j) / CPR & 63 : (l + 64 * j) / CPR, last);
+    // CPR == 4: the chunks of a lane are 16 rows apart and keep their (swizzled) column; otherwise the columns of chunk j
+    // and j + CPR are the same, and the stage holds the chunks in order
+    constexpr int NCOL = CPR == 4 ? 1 : CPR;
+    const uint8_t* srcc[NCOL];
+#pragma unroll
+    for (int j = 0; j < NCOL; ++j) srcc[j] = src + (l + 64 * j) % CPR * 16;
+    const uint32_t dst0 = smem_u32(sC) + (uint32_t)(CPR == 4 ? l / 4 * RB + code_chunk<CPR>(l & 3, l / 4) * 16 : l * 16);
     // sidecars: this lane's rows l and l + 64 (of the second matrix in a pair tile)
     constexpr int CKB = CodeStage<BITS>::CKB;
     const int64_t r0 = n0 + min(l, last), r1 = PAIR ? r0 : n0 + min(l + 64, last);
@@ -346,8 +353,8 @@ __device__ __forceinline__ bool load_codes(const uint32_t* codes, int64_t n0, in
         const uint32_t d = dst0 + (uint32_t)(buf * (128 * WT * RB));
 #pragma unroll
         for (int j = 0; j < NCH; ++j) {
-            const uint32_t dj = d + (CPR == 4 ? doff[0] + (uint32_t)(16 * j * RB) : doff[CPR == 4 ? 0 : j]);
-            const uint8_t* s = src + soff[j];
+            const uint32_t dj = d + (uint32_t)(j * 1024);
+            const uint8_t* s = row_at(srcc[j % NCOL], row[j], rowbytes);
             if (PAIR && j >= NCH / 2) s += second;
             const int col = CPR == 4 ? (l & 3) : (l + 64 * j) % CPR;
             if (col * 16 < rem) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dj), "l"(s) : "memory");
@@ -370,7 +377,8 @@ __device__ __forceinline__ bool load_codes(const uint32_t* codes, int64_t n0, in
             if (++slot == CD) slot = 0;
         }
         cp_async_arrive(cfull + buf);
-        src += RB;
+#pragma unroll
+        for (int j = 0; j < NCOL; ++j) srcc[j] += RB;
         rem -= RB;
         if (++buf == CD) { buf = 0; phase ^= 1u; }
     }

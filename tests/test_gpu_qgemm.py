@@ -193,3 +193,20 @@ def test_qgemm_weight_operand_is_rounded_once(bits, dtype):
         # the dequantizer rounds to float32 and then to 16 bits, the operand once: either neighbour of a tie
         ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
         assert torch.all((y.double() - exact).abs() <= exact.abs() * ulp * (1 + 1e-4) + 6.1e-8 * (dtype == torch.float16))
+
+
+@pytest.mark.parametrize("M", (16, 17))
+@pytest.mark.parametrize("bits,K", ((8, 34 << 20), (6, 46 << 20)))
+def test_rows_of_34_megabytes(bits, K, M):
+    """127 packed rows span more than 2^32 bytes: the last rows of a 128-row tile are the ones of their own product, bit
+    for bit (both take the same K split), in the GEMM and in the small-batch mat-vec."""
+    gs, N = 128, 128
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(bits)
+    wq = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K * bits // 32), generator=gen, device=DEV, dtype=torch.int32)
+    s = torch.rand((N, K // gs), generator=gen, device=DEV).bfloat16() * 1e-4
+    b = -s
+    x = torch.empty((M, K), dtype=torch.bfloat16, device=DEV).normal_(generator=gen)
+    y = jq.quantized_matmul(x, wq, s, b, group_size=gs, bits=bits)
+    assert torch.equal(y[:, 96:], jq.quantized_matmul(x, wq[96:], s[96:], b[96:], group_size=gs, bits=bits))
+    _lib.check(_lib.load().jq_device_status())
