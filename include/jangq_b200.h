@@ -240,7 +240,8 @@ int jq_gather_rows(const void* src, int64_t src_ld, const int32_t* order, const 
                    jq_stream_t stream);
 
 /* Grouped quantized GEMM over the expert-sorted rows (gather_qmm with sorted_indices=True):
- * y_sorted[p, :] = x_sorted[p, :] . deq(W[expert of row p])^T, on the tcgen05 tensor cores. */
+ * y_sorted[p, :] = x_sorted[p, :] . deq(W[expert of row p])^T, on the tcgen05 tensor cores.
+ * Of the tile list the first min(*num_tiles, max_tiles) entries are read. */
 int jq_moe_gemm(const void* x_sorted, int act_dtype, int64_t max_rows, int64_t ldx,
                 const int32_t* expert_offsets, const int32_t* tile_expert, const int32_t* tile_row0,
                 const int32_t* num_tiles, int64_t max_tiles, const uint32_t* const* codes_tab,

@@ -60,6 +60,7 @@ struct GemmArgs {
     const int32_t* tile_expert;
     const int32_t* tile_row0;
     const int32_t* num_tiles;
+    int max_tiles;                 // entries the caller stated the list to have: no more are read, whatever *num_tiles says
     const int32_t* expert_offsets;
     const uint32_t* const* codes_tab;
     const void* const* scales_tab;
@@ -484,7 +485,7 @@ qgemm_pers_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nkb = (int)(a.K / GEMM_BK), nst = (nkb + CKB - 1) / CKB;
     const int nx = (int)((a.N + (GU ? 63 : 127)) / (GU ? 64 : 128));
-    const int total = nx * *a.num_tiles * a.sub;
+    const int total = nx * min(*a.num_tiles, a.max_tiles) * a.sub;
     const int first = blockIdx.x, step = gridDim.x;
     if (first >= total) return;              // uniform for the CTA, before any barrier or tensor-memory allocation
 
@@ -813,6 +814,7 @@ int qgemm_dispatch(const void* x, int x_dtype, int64_t M, int64_t ldx, const uin
     a.tile_expert = grp ? grp->tile_expert : nullptr;
     a.tile_row0 = grp ? grp->tile_row0 : nullptr;
     a.num_tiles = grp ? grp->num_tiles : nullptr;
+    a.max_tiles = grp ? (int)std::min<int64_t>(grp->max_tiles, INT32_MAX) : 0;       // 65535 at most, checked below
     a.expert_offsets = grp ? grp->expert_offsets : nullptr;
     a.codes_tab = grp ? grp->codes_tab : nullptr;
     a.scales_tab = grp ? grp->scales_tab : nullptr;

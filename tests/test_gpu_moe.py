@@ -791,16 +791,18 @@ def test_combine_batches_of_eight_slots(k, D):
     assert torch.equal(out, ref)
 
 
-def grouped(x, sp, bank, tabs=None):
-    """jq_moe_gemm_tiled over every width of `bank`; tabs replaces its (scales, biases) pointer tables."""
+def grouped(x, sp, bank, tabs=None, max_tiles=None):
+    """jq_moe_gemm_tiled over every width of `bank`; tabs replaces its (scales, biases) pointer tables, max_tiles the
+    stated length of the tile list."""
     lib = _lib.load()
     dt = _lib.dtype_id(x.dtype)
     stab, btab = tabs or (bank.scales_tab, bank.biases_tab)
+    max_tiles = sp.max_tiles if max_tiles is None else max_tiles
     y = torch.full((x.shape[0] + 1, bank.N + 8), 7.0, dtype=x.dtype, device=DEV)
     for bits in bank.distinct_bits:
         _lib.check(lib.jq_moe_gemm_tiled(
             x.data_ptr(), dt, sp.n, x.stride(0), sp.offsets.data_ptr(), sp.tile_expert.data_ptr(), sp.tile_row0.data_ptr(),
-            sp.num_tiles.data_ptr(), sp.max_tiles, sp.tile_m, bank.codes_tab.data_ptr(), stab.data_ptr(), btab.data_ptr(),
+            sp.num_tiles.data_ptr(), max_tiles, sp.tile_m, bank.codes_tab.data_ptr(), stab.data_ptr(), btab.data_ptr(),
             bank.bits_tab.data_ptr() if bank.bits_tab is not None else None, dt, bank.N, bank.K, bits, bank.group_size,
             y.data_ptr(), y.stride(0), _lib.stream_ptr()))
     assert bool((y[:sp.n, bank.N:] == 7.0).all()) and bool((y[sp.n:] == 7.0).all())
@@ -850,4 +852,18 @@ def test_grouped_gemm_experts_of_mixed_sidecar_alignment(bits, K, gs):
         sp = SortedPairs(idx, E, tile_m=tile_m)
         assert torch.equal(grouped(x, sp, banks[0], tabs[:2]), grouped(x, sp, banks[0]))
         assert torch.equal(gate_up(x, sp, *banks, tabs), gate_up(x, sp, *banks))
+    _lib.check(_lib.load().jq_device_status())
+
+
+@pytest.mark.parametrize("tile_m", (128, 192))
+def test_grouped_gemm_reads_no_more_tiles_than_stated(tile_m):
+    """*num_tiles is on the device; of a list that it says is longer than max_tiles the surplus stays untouched."""
+    E, N, K = 4, 256, 128
+    bank, _ = make_bank(E, N, K, 4, 64, seed=3)
+    idx = torch.repeat_interleave(torch.arange(E, device=DEV, dtype=torch.int32), 2 * tile_m)      # two tiles per expert
+    x = torch.randn((idx.numel(), K), device=DEV).bfloat16()
+    sp = SortedPairs(idx, E, tile_m=tile_m)
+    want = grouped(x, sp, bank)
+    got = grouped(x, sp, bank, max_tiles=3)
+    assert torch.equal(got[:3 * tile_m], want[:3 * tile_m]) and bool((got[3 * tile_m:] == 7.0).all())
     _lib.check(_lib.load().jq_device_status())
