@@ -297,7 +297,8 @@ def quantized_matmul(x: torch.Tensor, w: torch.Tensor, scales: torch.Tensor, bia
     if x.dtype not in (torch.bfloat16, torch.float16):
         raise JangqError(_lib.JQ_EINVAL, f"activations must be bfloat16 or float16, got {x.dtype}")
     matrix = len(xshape) == 2
-    x2 = x if matrix else x.reshape(-1, K)
+    # the pitch of a single row is whatever the view it came from had (a transposed column has 1): a reshape sets it to K
+    x2 = x if matrix and (xshape[0] != 1 or x.stride(0) == K) else x.reshape(-1, K)
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
     M, N = x2.shape[0], w.shape[0]
