@@ -152,12 +152,16 @@ def dtype_id(dt: torch.dtype) -> int:
 
 # A small call is a few microseconds of kernel, so what Python does around it is what the caller waits for: the raw
 # stream handle instead of a Stream object, no device switch when the device is current already, integers instead of
-# torch.device objects in the checks.
+# torch.device objects in the checks.  Both functions are private to torch; its public ones serve where it lacks them.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+
+
 def stream_ptr(device=None) -> int:
-    if device is not None and not isinstance(device, torch.device):
-        device = torch.device("cuda", device) if isinstance(device, int) else torch.device(device)
-    index = None if device is None else device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    """Handle of the current stream of `device` (a torch.device, an ordinal, a string; None: the current device)."""
+    if _raw_stream is not None and isinstance(device, torch.device) and device.type == "cuda" and device.index is not None:
+        return _raw_stream(device.index)
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 _same_device = contextlib.nullcontext()
@@ -165,7 +169,7 @@ _same_device = contextlib.nullcontext()
 
 def on_device(dev: torch.device):
     """Context manager that makes `dev` (of a CUDA tensor, so CUDA is initialised) the current device."""
-    return _same_device if torch._C._cuda_getDevice() == dev.index else torch.cuda.device(dev)
+    return _same_device if _current_device() == dev.index else torch.cuda.device(dev)
 
 
 def require_cuda(*tensors: torch.Tensor) -> torch.device:

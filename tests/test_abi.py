@@ -58,3 +58,26 @@ def test_cpu_tensors_are_rejected():
     import jangq_b200 as jq
     with pytest.raises(_lib.JangqError):
         jq.quantize(torch.zeros(4, 64), 64, 4)
+
+
+def test_stream_handle_takes_what_torch_takes(monkeypatch):
+    """The raw handle is a short cut for a device with an ordinal; every other form, and a torch without the private
+    function, goes through torch.cuda.current_stream, which refuses devices that are not CUDA's."""
+    import torch
+    asked = []
+
+    def current_stream(device=None):
+        asked.append(device)
+        if isinstance(device, torch.device) and device.type != "cuda":
+            raise ValueError(f"Expected a cuda device, but got: {device}")
+        return type("Stream", (), {"cuda_stream": 7})()
+
+    monkeypatch.setattr(torch.cuda, "current_stream", current_stream)
+    monkeypatch.setattr(_lib, "_raw_stream", lambda index: 100 + index)
+    assert _lib.stream_ptr(torch.device("cuda", 3)) == 103 and not asked
+    forms = [None, 1, "cuda:1", torch.device("cuda")]
+    assert [_lib.stream_ptr(f) for f in forms] == [7] * 4 and asked == forms
+    with pytest.raises(ValueError):
+        _lib.stream_ptr(torch.device("cpu"))
+    monkeypatch.setattr(_lib, "_raw_stream", None)
+    assert _lib.stream_ptr(torch.device("cuda", 3)) == 7
