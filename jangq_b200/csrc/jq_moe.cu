@@ -369,7 +369,9 @@ __global__ void swiglu_kernel(const AT* __restrict__ g, const AT* __restrict__ u
 // out[t, :] = sum_j (w ? w[t*k+j] : 1) * y[inv ? inv[t*k+j] : t*k+j, :]  in f32, slots in order
 // (dsv41/model.py:1230-1234); pairs with inv < 0 (experts of another rank) are skipped.  `shared`
 // (optional, [T, D]) is the always-on expert's output, added to the routed sum in f32 (model.py:1237-1245).
-template <typename AT>
+// BATCH slots at a time: their row numbers first, then all their vectors, so that the loads of a batch are in flight
+// together (one after the other they are a chain of 2 k dependent loads).
+template <typename AT, int BATCH>
 __global__ void combine_kernel(const AT* __restrict__ y, int64_t ldy, const int32_t* __restrict__ inv,
                                const float* __restrict__ w, int T, int k, int D, AT* __restrict__ out, int64_t ldo,
                                float* __restrict__ out_f32, const AT* __restrict__ shared, int64_t ld_shared) {
@@ -384,18 +386,16 @@ __global__ void combine_kernel(const AT* __restrict__ y, int64_t ldy, const int3
                 float acc[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-                // eight slots at a time: their row numbers first, then all their vectors, so that the loads of a
-                // batch are in flight together (one after the other they are a chain of 2 k dependent loads)
-                for (int j0 = 0; j0 < k; j0 += 8) {
-                    int p[8];
-                    uint4 q[8];
+                for (int j0 = 0; j0 < k; j0 += BATCH) {
+                    int p[BATCH];
+                    uint4 q[BATCH];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) p[j] = j0 + j < k ? (inv ? inv[t * k + j0 + j] : t * k + j0 + j) : -1;
+                    for (int j = 0; j < BATCH; ++j) p[j] = j0 + j < k ? (inv ? inv[t * k + j0 + j] : t * k + j0 + j) : -1;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
+                    for (int j = 0; j < BATCH; ++j)
                         if (p[j] >= 0) q[j] = __ldg(reinterpret_cast<const uint4*>(y + (int64_t)p[j] * ldy + c));
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                    for (int j = 0; j < BATCH; ++j) {
                         if (p[j] < 0) continue;
                         const float wj = w ? w[t * k + j0 + j] : 1.0f;
                         const AT* ya = reinterpret_cast<const AT*>(&q[j]);
@@ -1043,10 +1043,21 @@ int jq_moe_combine_shared(const void* y, int64_t ldy, const int32_t* inv, const 
     JQ_REQUIRE(y && (out || out_f32), JQ_EINVAL, "null pointer");
     JQ_REQUIRE(shared_y == nullptr || ld_shared >= D, JQ_EINVAL, "leading dimension of the shared expert's rows too small");
     const int blocks = (int)(T < 8 * 148 ? T : 8 * 148);
-    JQ_DISPATCH_DTYPE16(dtype, A,
-        (combine_kernel<A><<<blocks, 256, 0, (cudaStream_t)stream>>>((const A*)y, ldy, inv, weights, (int)T, k, (int)D,
-                                                                      (A*)out, ldo, out_f32, (const A*)shared_y,
-                                                                      ld_shared)))
+    // Slots per batch: k in the fewest equal parts of at most six, or eight where every CTA has an SM of its own (its
+    // registers cost nothing there).  Eight predicated slots for any k took up to 1.9 times as long as one after the
+    // other at k = 1 and 2 (16384 tokens x 7168, k = 1: 112 -> 159 us, now 112; k = 2: 181, 183, 138), and at 512
+    // tokens a part of eight gave nothing over single slots (x 4096, k = 8: 7.1, 6.8, in parts of four 5.7).
+    const int cap = T <= sm_count() ? 8 : 6, parts = (k + cap - 1) / cap;
+#define JQ_COMBINE(B)                                                                                              \
+    case B:                                                                                                        \
+        JQ_DISPATCH_DTYPE16(dtype, A,                                                                              \
+            (combine_kernel<A, B><<<blocks, 256, 0, (cudaStream_t)stream>>>(                                       \
+                (const A*)y, ldy, inv, weights, (int)T, k, (int)D, (A*)out, ldo, out_f32, (const A*)shared_y, ld_shared))) \
+        break;
+    switch ((k + parts - 1) / parts) {
+        JQ_COMBINE(1) JQ_COMBINE(2) JQ_COMBINE(3) JQ_COMBINE(4) JQ_COMBINE(5) JQ_COMBINE(6) JQ_COMBINE(7) JQ_COMBINE(8)
+    }
+#undef JQ_COMBINE
     return check_launch("moe_combine");
 }
 

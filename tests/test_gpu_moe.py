@@ -770,12 +770,13 @@ def test_topk_over_every_register_count(E, dtype):
     assert torch.all((w.double() - ref).abs() <= 1e-5 * ref)
 
 
-@pytest.mark.parametrize("k", (1, 7, 8, 9, 17))
+@pytest.mark.parametrize("T", (5, 300))
+@pytest.mark.parametrize("k", (1, 2, 3, 4, 5, 6, 7, 8, 9, 13, 17))
 @pytest.mark.parametrize("D", (8, 264, 2048))
-def test_combine_batches_of_eight_slots(k, D):
-    """Slots are loaded eight at a time and added in slot order: the float32 sums of the plain loop, bit for bit."""
+def test_combine_batches_of_slots(k, D, T):
+    """Slots are loaded in batches of one to eight (six with many tokens) and added in slot order: the float32 sums of the
+    plain loop, bit for bit."""
     lib = _lib.load()
-    T = 5
     gen = torch.Generator(device=DEV)
     gen.manual_seed(k + D)
     y = torch.randn((T * k, D), generator=gen, device=DEV).to(torch.bfloat16)
