@@ -248,9 +248,9 @@ int jq_moe_gemm(const void* x_sorted, int act_dtype, int64_t max_rows, int64_t l
                 const void* const* scales_tab, const void* const* biases_tab, const int32_t* bits_tab,
                 int sidecar_dtype, int64_t N, int64_t K, int bits, int group_size, void* y_sorted,
                 int64_t ldy, jq_stream_t stream);
-/* jq_moe_gemm over a tile list of tile_m rows per entry (the tile_m given to jq_moe_sort): 128, 192 -- the largest tile
- * that one pass over an expert's weights serves -- or 256 (two tiles of 128; bf16 activations and N >= 256 only,
- * JQ_EUNSUPPORTED otherwise). */
+/* jq_moe_gemm over a tile list of tile_m rows per entry (the tile_m given to jq_moe_sort): 128, 192 or 256 (bf16
+ * activations and N >= 256 only, JQ_EUNSUPPORTED otherwise).  One pass over an expert's weights serves a tile; a tile of
+ * up to 192 rows is stored while the next one is computed. */
 int jq_moe_gemm_tiled(const void* x_sorted, int act_dtype, int64_t max_rows, int64_t ldx,
                       const int32_t* expert_offsets, const int32_t* tile_expert, const int32_t* tile_row0,
                       const int32_t* num_tiles, int64_t max_tiles, int tile_m, const uint32_t* const* codes_tab,

@@ -50,7 +50,6 @@ struct GemmArgs {
     int64_t M, N, K, ldy;
     int gs, G;
     int tn;          // activation rows per tile (multiple of 16, <= TNMAX)
-    int sub;         // grouped mode: tiles of tn rows per entry of the tile list
     int box_rows;    // activation rows per TMA box: tn, or 32 when the rows of a tile vary (grouped mode)
     int y_pair_ok;   // rows of y are 4-byte aligned
     int y_vec_ok;    // rows of y are 8-byte aligned
@@ -411,16 +410,19 @@ qgemm_ts_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
 }
 
 // ---- persistent form --------------------------------------------------------------------------------------
-// One CTA per SM walks tiles of 128 weight rows x up to 192 activation rows (blockIdx.x, + gridDim.x, ...).  Two
-// accumulators of 192 columns and four A slots fill the tensor memory: while the epilogue warps store one tile, the
-// MMAs fill the other accumulator, and copies and expansion of the next tile start before this one's MMAs are done.
+// One CTA per SM walks tiles of 128 weight rows x up to TN activation rows (blockIdx.x, + gridDim.x, ...).  TN = 192: two
+// accumulators and four A slots fill the tensor memory; while the epilogue warps store one tile, the MMAs fill the other
+// accumulator, and copies and expansion of the next tile start before this one's MMAs are done.  TN = 256 (tile lists of
+// 256 rows): one accumulator, so the next tile's MMAs wait until this one is read, but its four A slots are full by then;
+// one expansion of a weight tile serves 256 rows (as two tiles of 128 they were expanded twice: 8192 rows over 8
+// experts, 2048x4096 2-bit 185 us, now 134).
 // Without it every 128-row tile of an expert paid 5.5 us of start and epilogue for 12 to 64 k-blocks of 0.3 us, and a
 // grid sized for the largest possible tile list started thousands of CTAs that had nothing to do.
 // GU (grouped mode): the tile's 128 weight rows are 64 rows of the gate projection and the same 64 rows of the up
 // projection, so both sums of an output meet in one CTA: the epilogue exchanges them through shared memory in f32 and
 // stores h.  Gate and up results never go through memory, and one launch replaces three.
-template <int BITS> struct PersCfg {
-    static constexpr int TNMAX = 192, ND = 2, RA = 4, NCOLS = 512, NKG = RA;
+template <int BITS, int TN> struct PersCfg {
+    static constexpr int TNMAX = TN, ND = TN == 192 ? 2 : 1, RA = 4, NCOLS = 512, NKG = RA;
     static constexpr int ACOL = ND * TNMAX;
     static constexpr int CKB = CodeStage<BITS>::CKB, RB = CodeStage<BITS>::RB, CD = 6;
     static constexpr int C_STAGE = 128 * RB, X_STAGE = TNMAX * GEMM_BK * 2;
@@ -428,9 +430,10 @@ template <int BITS> struct PersCfg {
     static constexpr int NBAR = 2 * RA + 2 * CD + 2 * ND;
     static constexpr int SIDE_OFF = RA * X_STAGE + CD * C_STAGE;
     static constexpr int SW_OFF = SIDE_OFF + CD * SIDE_SLOT;             // float[32][128]: gate/up exchange
-    static constexpr int WT_OFF = SW_OFF + 32 * 128 * 4;                 // float[192]: routing weights of the tile's rows
+    static constexpr int WT_OFF = SW_OFF + 32 * 128 * 4;                 // float[TN]: routing weights of the tile's rows
     static constexpr int BAR_OFF = WT_OFF + TNMAX * 4;
     static constexpr size_t SMEM = 1024 + BAR_OFF + NBAR * 8 + 16;
+    static_assert(ACOL + RA * 32 <= NCOLS, "accumulators and A slots fit the tensor memory");
 };
 
 struct PersTile {
@@ -445,9 +448,8 @@ __device__ __forceinline__ PersTile pers_tile(const GemmArgs& a, int tile, int n
     PersTile t;
     const int bx = tile % nx, by = tile / nx;
     t.n0 = (int64_t)bx * (GU ? 64 : 128);
-    const int entry = by / a.sub, part = by - entry * a.sub;
-    const int e = a.tile_expert[entry];
-    t.m0 = (int64_t)a.tile_row0[entry] + (int64_t)part * a.tn;
+    const int e = a.tile_expert[by];
+    t.m0 = a.tile_row0[by];
     int64_t m_end = a.expert_offsets[e + 1];
     t.codes = a.codes_tab[e]; t.scales = a.scales_tab[e]; t.biases = a.biases_tab[e];
     t.codes2 = nullptr; t.scales2 = nullptr; t.biases2 = nullptr;
@@ -464,10 +466,10 @@ template <bool GU> __device__ __forceinline__ int pers_side_mode(const GemmArgs&
     return m == 0 || m2 == 0 ? 0 : max(m, m2);               // the copy that both matrices are aligned for
 }
 
-template <typename AT, int BITS, bool GU>
-__global__ void __launch_bounds__(PersCfg<BITS>::THREADS, 1)
+template <typename AT, int BITS, bool GU, int TN>
+__global__ void __launch_bounds__(PersCfg<BITS, TN>::THREADS, 1)
 qgemm_pers_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
-    using C = PersCfg<BITS>;
+    using C = PersCfg<BITS, TN>;
     constexpr int CKB = C::CKB, RB = C::RB, CD = C::CD, RA = C::RA, NKG = C::NKG;
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -485,7 +487,7 @@ qgemm_pers_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nkb = (int)(a.K / GEMM_BK), nst = (nkb + CKB - 1) / CKB;
     const int nx = (int)((a.N + (GU ? 63 : 127)) / (GU ? 64 : 128));
-    const int total = nx * min(*a.num_tiles, a.max_tiles) * a.sub;
+    const int total = nx * min(*a.num_tiles, a.max_tiles);
     const int first = blockIdx.x, step = gridDim.x;
     if (first >= total) return;              // uniform for the CTA, before any barrier or tensor-memory allocation
 
@@ -744,11 +746,11 @@ static int launch_gemm(const CUtensorMap& xmap, const GemmArgs& a, int64_t m_til
     return check_launch("qgemm");
 }
 
-template <typename AT, int BITS, bool GU>
+template <typename AT, int BITS, bool GU, int TN>
 static int launch_pers(const CUtensorMap& xmap, const GemmArgs& a, int64_t m_tiles, cudaStream_t st) {
-    using C = PersCfg<BITS>;
+    using C = PersCfg<BITS, TN>;
     static_assert(C::SMEM <= GEMM_SMEM, "shared memory of one CTA");
-    auto kernel = qgemm_pers_kernel<AT, BITS, GU>;
+    auto kernel = qgemm_pers_kernel<AT, BITS, GU, TN>;
     static bool attr_done[64] = {};
     int dev = 0;
     JQ_CUDA_OK(cudaGetDevice(&dev));
@@ -832,10 +834,9 @@ int qgemm_dispatch(const void* x, int x_dtype, int64_t M, int64_t ldx, const uin
     if (grp) {
         JQ_REQUIRE(grp->tile_m == 128 || grp->tile_m == 192 || (grp->tile_m == 256 && N >= 256 && x_dtype == JQ_BF16),
                    JQ_EUNSUPPORTED, "tile lists of 256 rows need bf16 activations and N >= 256 (128 or 192 otherwise)");
-        a.tn = grp->tile_m == 192 ? 192 : 128;
-        a.sub = grp->tile_m / a.tn;
+        a.tn = grp->tile_m;
         a.box_rows = 32;
-        m_tiles = grp->max_tiles * a.sub;
+        m_tiles = grp->max_tiles;
     } else {
         // The number of row tiles (nt, of tn rows each) and the K split with the shortest estimated time.  Measured on
         // B200 over M = 17 .. 4096: a CTA walks a k-block in 0.20 + 0.0006 tn us (the expansion of the codes sets the
@@ -858,7 +859,6 @@ int qgemm_dispatch(const void* x, int x_dtype, int64_t M, int64_t ldx, const uin
                 if (t < best) { best = t; m_tiles = tiles; a.tn = (int)tn; ks = S; }
             }
         }
-        a.sub = 1;
         a.box_rows = a.tn;
     }
     if (m_tiles == 0) return JQ_OK;
@@ -877,14 +877,17 @@ int qgemm_dispatch(const void* x, int x_dtype, int64_t M, int64_t ldx, const uin
 
 #define JQ_GEMM_T(T, B)                                                                                   \
     {                                                                                                     \
-        if (gu) return launch_pers<T, B, true>(xmap, a, m_tiles, st);                                     \
-        if (grp) return launch_pers<T, B, false>(xmap, a, m_tiles, st);                              \
+        if (gu) return launch_pers<T, B, true, 192>(xmap, a, m_tiles, st);                                \
+        if (grp) return launch_pers<T, B, false, 192>(xmap, a, m_tiles, st);                              \
         if (ks == 4) return launch_gemm<T, B, 4>(xmap, a, m_tiles, st);                                   \
         if (ks == 2) return launch_gemm<T, B, 2>(xmap, a, m_tiles, st);                                   \
         return launch_gemm<T, B, 1>(xmap, a, m_tiles, st);                                                \
     }
 #define JQ_GEMM_CASE(B)                                                                                   \
     if (bits == B) {                                                                                      \
+        if (grp && grp->tile_m == 256)                         /* bf16 only, see above */                 \
+            return gu ? launch_pers<__nv_bfloat16, B, true, 256>(xmap, a, m_tiles, st)                    \
+                      : launch_pers<__nv_bfloat16, B, false, 256>(xmap, a, m_tiles, st);                  \
         if (x_dtype == JQ_BF16) JQ_GEMM_T(__nv_bfloat16, B)                                               \
         JQ_GEMM_T(__half, B)                                                                              \
     }

@@ -868,3 +868,23 @@ def test_grouped_gemm_reads_no_more_tiles_than_stated(tile_m):
     got = grouped(x, sp, bank, max_tiles=3)
     assert torch.equal(got[:3 * tile_m], want[:3 * tile_m]) and bool((got[3 * tile_m:] == 7.0).all())
     _lib.check(_lib.load().jq_device_status())
+
+
+@pytest.mark.parametrize("bits", (2, 3, 4, 5, 6, 8))
+@pytest.mark.parametrize("K", (640, 1152))
+def test_grouped_gemm_of_256_row_tiles(bits, K):
+    """Tile lists of 256 rows (one accumulator) against 192 and 128: the same sums in the same order, bit for bit, over
+    experts whose last tile holds 1, 16, 17, 128, 129, 192, 193 and 256 rows, several tiles per CTA."""
+    counts = (1, 16, 17, 128, 129, 192, 193, 256, 0, 257, 500) * 2
+    E, N = len(counts), 1200
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(bits + K)
+    gate, up = (jq.ExpertBank(*jq.quantize((torch.randn((E, N, K), generator=gen, device=DEV) * 0.1).bfloat16(), 64, bits), bits, 64)
+                for _ in range(2))
+    idx = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)]).to(DEV)
+    x = torch.randn((idx.numel(), K), generator=gen, device=DEV).bfloat16()
+    lists = [SortedPairs(idx, E, tile_m=m) for m in (256, 192, 128)]
+    plain = [grouped(x, sp, gate) for sp in lists]
+    fused = [gate_up(x, sp, gate, up) for sp in lists]
+    assert all(torch.equal(plain[0], p) for p in plain[1:]) and all(torch.equal(fused[0], f) for f in fused[1:])
+    _lib.check(_lib.load().jq_device_status())
