@@ -526,11 +526,18 @@ int qgemv_dispatch_items(const void* x, int x_dtype, int64_t M, int64_t ldx, con
     if (live.count == 0) return JQ_OK;
     const int kern = gemv_kernel_choice();
     // More than eight rows: one launch of the small-batch tensor-memory kernel instead of two of eight rows (16 rows,
-    // 14336x4096 4-bit 26 us against 52).  It also takes 8-bit codes from six rows on, where the limbs of the other
-    // tensor-memory kernel outgrow 16 columns (8 rows: 14336x4096 23 us against 30, 4096x4096 11.8 against 14.7; five
-    // rows tie).  At eight rows of narrower codes it ties or loses (4-bit 24.5 against 23.7 us, 2-bit 4096x4096 11.5
-    // against 9.6).
-    int64_t step = fast && kern == 0 && (M > 8 || (bits == 8 && M > 5)) ? 16 : 8;
+    // 14336x4096 4-bit 26 us against 52).  At six to eight rows of 8-bit codes, where the limbs of the other tensor-memory
+    // kernel outgrow 16 columns, the shorter estimate decides: in one round of CTAs with groups of 128 that kernel still
+    // wins (6 rows, 14336x4096: 18.6 us against 21.7), otherwise this one does (groups of 64 21.8 against 23.5, 22016x4096 33.5
+    // against 38.7, 2432x4096 10 against 21.6).  At eight rows of narrower codes it ties or loses (4-bit 24.5 against
+    // 23.7 us, 2-bit 4096x4096 11.5 against 9.6).
+    int64_t step = 8;
+    if (fast && kern == 0 && M > 8) step = 16;
+    if (fast && kern == 0 && bits == 8 && M > 5 && M <= 8) {
+        int64_t blocks = 0;
+        for (int i = 0; i < live.count; ++i) blocks += (live.N[i] + 127) / 128;
+        if (ts_split(blocks, K).us <= tc_estimate_us(blocks, K, gs, M, x_dtype)) step = 16;
+    }
     for (int64_t m0 = 0; m0 < M; m0 += step) {
         GemvArgs a = {};
         a.x = (const char*)x + m0 * ldx * dtype_size(x_dtype);

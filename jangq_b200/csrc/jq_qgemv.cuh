@@ -168,7 +168,13 @@ int launch_pint_kernel(const GemvArgs& a, const GemvBatch& bt, int act_dtype, in
 int launch_tc_kernel(const GemvArgs& a, const GemvBatch& bt, int act_dtype, int bits, int gs, cudaStream_t st,
                      bool* launched);
 
+// Estimated time (us) of that kernel for six to eight rows of 8-bit codes; very large where it does not run well.
+float tc_estimate_us(int64_t row_blocks, int64_t K, int gs, int64_t M, int act_dtype);
+
 // small-batch kernel (jq_qgemv_ts.cu): up to 16 activation rows in one launch, any width but 5; same convention
+struct TsSplit { int S; float us; };
+TsSplit ts_split(int64_t row_blocks, int64_t K);
+int resident_clusters(int S, int per_sm);
 int launch_ts_kernel(const GemvArgs& a, const GemvBatch& bt, int act_dtype, int bits, int gs, cudaStream_t st,
                      bool* launched);
 

@@ -543,6 +543,15 @@ static int launch_cfg(const TcMaps& maps, GemvArgs a, GemvBatch bt, int S, int n
     return JQ_OK;
 }
 
+// Few row blocks (at most one CTA per SM): the largest cluster of up to eight that gives every SM at most one CTA
+static int spread(int64_t row_blocks, int nquads) {
+    const int sms = sm_count();
+    int S = 1;
+    if (row_blocks <= sms)
+        while (S < 8 && S < nquads && row_blocks * (S + 1) <= sms) ++S;
+    return S;
+}
+
 // Cluster size and ring depth.
 //   * Few row blocks (at most one CTA per SM): the largest S <= 8 that still gives every SM at most one
 //     CTA; the ring then holds the CTA's whole K slice where it fits, so that all of the matrix is in
@@ -553,14 +562,10 @@ static int launch_shape(const TcMaps& maps, const GemvArgs& a, const GemvBatch& 
     constexpr int TPQ = 4 * GS / TK;
     using RG = Ring<BITS, GS, NCOL>;
     constexpr int TPS = BITS == 8 ? 2 : 8 / BITS;          // tiles per stage
-    const int sms = sm_count();
     const int nquads = a.G / 4;
     int64_t row_blocks = 0;
     for (int i = 0; i < bt.count; ++i) row_blocks += (bt.N[i] + ROWS - 1) / ROWS;
-    int S = 1;
-    if (row_blocks <= sms) {
-        while (S < 8 && S < nquads && row_blocks * (S + 1) <= sms) ++S;
-    }
+    int S = spread(row_blocks, nquads);
     auto fit_ns = [&](int s_) {
         const int sq_max = (nquads + s_ - 1) / s_;
         const int want = (sq_max * TPQ + TPS - 1) / TPS;      // stages of the longest slice
@@ -585,6 +590,20 @@ static int launch_shape(const TcMaps& maps, const GemvArgs& a, const GemvBatch& 
 
 }  // namespace tcv
 
+// One round of CTAs, each with a slice of K of at most 4096 codes (the limbs of a longer one crowd out the ring: 14336 x 11264,
+// 6 rows, 133 us): 2.6 us and 0.25 to 0.35 us per 64 codes by group size, type and rows (short slices 4.6 and 0.19), plus the
+// sum over a cluster.
+// Measured on B200, 4 to 148 row blocks, K = 2048 to 11264.
+float tc_estimate_us(int64_t row_blocks, int64_t K, int gs, int64_t M, int act_dtype) {
+    const int nquads = (int)(K / gs / 4), S = tcv::spread(row_blocks, nquads);
+    const int64_t slice = (int64_t)((nquads + S - 1) / S) * 4 * gs;
+    if (slice > 4096 || row_blocks > resident_clusters(S, 1)) return 1e30f;
+    const float r = (float)(M - 6);
+    const float per64 = gs == 128 ? 0.25f + 0.015f * r : act_dtype == JQ_F16 ? 0.285f + 0.0165f * r : 0.3275f + 0.0125f * r;
+    const float sum = S == 1 ? 0.f : (S == 2 ? 1.6f : S < 5 ? (float)S - 0.3f : 5.5f) + (gs == 64 ? 1.5f : 0.f);
+    const float k = (float)(slice / 64), walk = k * per64 + 2.6f, least = k * 0.19f + 4.6f;
+    return (walk > least ? walk : least) + sum;
+}
 
 // Dense mat-vecs (one launch for all matrices of `bt`) on the tensor-memory kernel; *launched stays
 // false when the shape does not fit it.

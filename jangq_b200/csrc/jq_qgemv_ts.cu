@@ -17,6 +17,8 @@
 // Every mbarrier wait is bounded; a wait that runs out sets the status word and the CTA leaves through the common exit.
 #include <cuda.h>
 
+#include <atomic>
+
 #include "jq_qgemv.cuh"
 #include "jq_ts.cuh"
 
@@ -208,7 +210,7 @@ qgemv_ts_kernel(const __grid_constant__ CUtensorMap xmap, const GemvArgs a, cons
                 for (int h = 0; h < 2; ++h) {                    // 32 codes at a time keep the registers for two CTAs per SM
                     uint32_t cur[BITS], out[16];
                     load_codes32<BITS, CPR>(crow, r, kbi, h, cur);
-                    dequant_fast<AT, BITS, 1>(cur, TsExact<AT>::C, 0u, out);
+                    dequant_fast<AT, BITS, 1, true>(cur, TsExact<AT>::C, 0u, out);
                     tmem_st16(lane_base + (uint32_t)(t * 32 + h * 16), out);
                 }
                 tmem_st_wait();
@@ -320,6 +322,60 @@ static int launch(const CUtensorMap& xmap, GemvArgs a, GemvBatch bt, int S, cuda
 
 }  // namespace tsv
 
+// Stands for a kernel whose shared memory decides how many CTAs an SM holds; never launched.  (Asked about the mat-vec kernel
+// itself, whose thirteen warps of 72 registers fit an SM twice, the query says once.)
+static __global__ void residency_kernel() {}
+
+// Clusters of S CTAs that the GPU holds at once with per_sm (1 or 2) CTAs on an SM.  Fewer than sms * per_sm / S: a cluster
+// stays inside a processing cluster whose SMs S need not divide (of 148 SMs: 45 threes, 33 fours, 15 eights; 93, 71, 33).
+int resident_clusters(int S, int per_sm) {
+    static std::atomic<int> cached[64][9][3];              // 0: not asked yet; host threads may ask twice
+    const int even = sm_count() * per_sm / S;
+    int dev = 0;
+    if (S <= 1 || S > 8 || per_sm < 1 || per_sm > 2 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return even;
+    int n = cached[dev][S][per_sm].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    constexpr int MOST = 200 * 1024;                       // over half of an SM's shared memory: one CTA each
+    auto kernel = residency_kernel;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)S * 1024u);               // the answer is no larger than the grid
+    cfg.blockDim = dim3(tsv::THREADS);
+    cfg.dynamicSmemBytes = per_sm == 1 ? MOST : MOST / 2;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        n = even;
+    }
+    cached[dev][S][per_sm].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+// Cluster size along K with the shortest estimated time (us): of two CTAs on an SM each walks a k-block in 0.52 us and
+// a round of them starts and ends in 3.6 us, one alone takes 0.33 and 4.4, and a split adds the exchange of the sums, more
+// with every round.  Measured on B200 over 4 to 460 row blocks, 2- to 8-bit codes, 6 to 16 rows (all scale alike).  The
+// largest split that one round holds, as before, left half of the chip idle between one and 1.4 row blocks per SM (9 rows,
+// 22016x4096 2-bit, group 128: 40.5 us unsplit, 36.5 by 3; 16 rows, 9600x11264 6-bit: 66.5 by 2, 48.7 by 3).
+TsSplit ts_split(int64_t row_blocks, int64_t K) {
+    TsSplit best = {1, 1e30f};
+    const int64_t chunks = K / 256;                        // of four k-blocks: what a split deals out
+    for (int S : {1, 2, 3, 4, 8}) {
+        if (chunks < S) break;
+        const int64_t one = resident_clusters(S, 1), two = resident_clusters(S, 2), rest = row_blocks % two;
+        const float pairs = (float)(row_blocks / two + (rest > one ? 1 : 0)), single = rest > 0 && rest <= one ? 1.f : 0.f;
+        const float k = (float)((chunks + S - 1) / S) * 4.f;
+        const float exchange = S == 1 ? 0.f : S == 2 ? 1.0f : S == 3 ? 2.5f : S == 4 ? 1.3f : 2.0f;
+        const float us = pairs * (0.52f * k + 3.6f) + single * (0.33f * k + 4.4f) + exchange * (0.4f + 0.6f * (pairs + single)) +
+                         (S >= 4 ? 0.6f * pairs : 0.f);
+        if (us < best.us) best = {S, us};
+    }
+    return best;
+}
+
 // Dense mat-vecs of up to 16 activation rows (a.M may exceed the 8 rows of the other kernels), one launch for all
 // matrices of `bt`; *launched stays false when the shape does not fit it.
 int launch_ts_kernel(const GemvArgs& a0, const GemvBatch& bt, int act_dtype, int bits, int gs, cudaStream_t st,
@@ -341,11 +397,7 @@ int launch_ts_kernel(const GemvArgs& a0, const GemvBatch& bt, int act_dtype, int
     a.gs_shift = gs == 128 ? 1 : 0;
     int64_t row_blocks = 0;
     for (int i = 0; i < bt.count; ++i) row_blocks += (bt.N[i] + tsv::ROWS - 1) / tsv::ROWS;
-    // K split: the largest that still fits one wave of two CTAs per SM, with at least four k-blocks each (14336x4096 4-bit,
-    // 16 rows: 31.5 us unsplit, 26.5 by 2, 31.1 by 4; 4096x4096 6-bit: 33.6, 20.4 by 2, 13.7 by 4, 14.0 by 8)
-    int S = 1;
-    const int64_t slots = 2 * (int64_t)sm_count();
-    while (S < 8 && row_blocks * (2 * S) <= slots && a.K / 64 / (2 * S) >= 4) S *= 2;
+    const int S = ts_split(row_blocks, a.K).S;
     int rc = JQ_OK;
 #define JQ_TS_CASE(B)                                                                                     \
     if (bits == B) {                                                                                      \

@@ -127,8 +127,9 @@ __device__ __forceinline__ void dequant_stream(const uint32_t (&u)[H * BITS], ui
 // 32*H codes of one row -> 16*H registers of two weights in k order, every weight rn(q*s + bias).
 // Fields of a word are taken two at a time, 16 bits apart, where they stand (or after one shift of the word), and the
 // results are put in k order by a byte permute: 13 instructions per 8 codes at 4 bits, 27 per 16 at 2 bits, 4 per 4 at
-// 8 bits (24, 48 and 14 with the exponent insert + subtract of dequant_pair).
-template <typename AT, int BITS, int H>
+// 8 bits (24, 48 and 14 with the exponent insert + subtract of dequant_pair).  EXACT: s is a power of two and b2 zero, so
+// nothing is rounded, and the 1024 that an 8-bit code of float16 carries leaves in the multiply-add.
+template <typename AT, int BITS, int H, bool EXACT = false>
 __device__ __forceinline__ void dequant_fast(const uint32_t (&u)[H * BITS], float s, uint32_t b2, uint32_t (&out)[16 * H]) {
     using A = Act<AT>;
     using P = P2<AT>;
@@ -143,11 +144,12 @@ __device__ __forceinline__ void dequant_fast(const uint32_t (&u)[H * BITS], floa
                 out[2 * i + 1] = P::fma(prmt(u[i], 0u, 0x4342), sp, b2);
             }
         } else {
-            const uint32_t sp = A::pack_hi(s, s);
+            const uint32_t sp = A::pack_hi(s, s), off = A::pack_hi(-1024.0f * s, -1024.0f * s);
 #pragma unroll
             for (int i = 0; i < 8 * H; ++i) {      // 0x64qq = 1024 + q
-                out[2 * i] = P::fma(P::sub(prmt(u[i], 0x64646464u, 0x4140), A::MAGIC), sp, b2);
-                out[2 * i + 1] = P::fma(P::sub(prmt(u[i], 0x64646464u, 0x4342), A::MAGIC), sp, b2);
+                const uint32_t v0 = prmt(u[i], 0x64646464u, 0x4140), v1 = prmt(u[i], 0x64646464u, 0x4342);
+                out[2 * i] = EXACT ? P::fma(v0, sp, off) : P::fma(P::sub(v0, A::MAGIC), sp, b2);
+                out[2 * i + 1] = EXACT ? P::fma(v1, sp, off) : P::fma(P::sub(v1, A::MAGIC), sp, b2);
             }
         }
     } else if constexpr (BITS == 4) {

@@ -422,10 +422,10 @@ def test_row_formed_in_the_launch_validation():
 @pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
 @pytest.mark.parametrize("bits", (2, 3, 4, 6, 8))
 @pytest.mark.parametrize("M,N,K,gs", ((6, 129, 256, 64), (8, 1, 512, 128), (9, 127, 1024, 64), (16, 300, 2304, 64),
-                                      (13, 4096, 2048, 128), (16, 40000, 256, 64)))
+                                      (13, 4096, 2048, 128), (16, 40000, 256, 64), (9, 9600, 2304, 64), (11, 1300, 768, 64)))
 def test_small_batch_kernel(M, N, K, gs, bits, dtype):
-    """More than eight rows (six for 8-bit codes) in one launch: one to 36 k-blocks, K split over 1 to 8 CTAs, ragged row
-    tiles.  Codes are exact and scales unrounded, so against float64 only the float32 sums (1e-5 of the largest output)
+    """More than eight rows (six for 8-bit codes) in one launch: four to 36 k-blocks, K split over 1, 2, 3, 4 and 8 CTAs (on
+    148 SMs), ragged row tiles.  Codes are exact and scales unrounded, so against float64 only the float32 sums (1e-5 of the largest output)
     and the output's rounding remain."""
     gen = torch.Generator(device="cuda:0")
     gen.manual_seed(M * 7 + bits)
