@@ -19,6 +19,7 @@ kernel; groups it does not take (other widths) keep their own launch.
 """
 from __future__ import annotations
 
+import os
 from typing import Sequence
 
 import torch
@@ -61,7 +62,7 @@ class GemvPlan:
         for g in self.groups:
             if any(self.x[i] is not self.x[g[0]] for i in g):
                 raise _lib.JangqError(_lib.JQ_EINVAL, "the linears of a group must read the same input buffer")
-        self.launches_per_run = sum(self._launches_of(g) * self._row_steps(g, m) for g in self.groups)
+        self.launches_per_run = sum(self._launches_of(g) for g in self.groups)
         # persistent: segments = ("program", StreamProgram) or ("groups", [group, ...]) in execution order
         self.persistent = bool(persistent) and m == 1
         self._segments = None
@@ -91,22 +92,33 @@ class GemvPlan:
         e = lin.scales.element_size()
         return n * k * lin.bits // 8 + n * (k // lin.group_size) * 2 * e + m * k * 2 + m * n * 2
 
-    def _row_steps(self, group, m: int) -> int:
-        """Launches per matrix run for m rows: one up to 8 rows, and up to 16 where the small-batch kernel fits."""
-        lin = self.linears[group[0]]
-        fits = lin.bits != 5 and lin.group_size in (64, 128) and (lin.in_features // lin.group_size) % 4 == 0
-        return 1 if m <= 8 or fits else (m + 7) // 8
-
     def _launches_of(self, group) -> int:
-        """Kernel launches of one group: runs of up to 4 consecutive members with equal (K, bits, group size)."""
-        n, run, prev = 0, 0, None
-        for i in group:
-            lin = self.linears[i]
-            key = (lin.in_features, lin.bits, lin.group_size)
-            if key != prev or run == 4:
-                n, run, prev = n + 1, 0, key
-            run += 1
+        """Kernel launches of one group.  A call takes up to QGEMV_MAX_BATCH members; in it, consecutive ones with equal
+        (K, bits, group size) go in runs of up to four, eight rows a launch or sixteen with the small-batch kernel; what
+        only the general kernel takes goes matrix by matrix, eight rows a launch (qgemv_dispatch_items)."""
+        n, run, prev = 0, [], None
+        for j, i in enumerate(list(group) + [None]):
+            lin = self.linears[i] if i is not None else None
+            key = (lin.in_features, lin.bits, lin.group_size) if lin is not None else None
+            if run and (key != prev or len(run) == 4 or j % _lib.QGEMV_MAX_BATCH == 0):
+                n += self._launches_of_run(run)
+                run = []
+            if lin is not None:
+                run.append(lin)
+            prev = key
         return n
+
+    def _launches_of_run(self, run) -> int:
+        steps = (self.m + 7) // 8
+        l0 = run[0]
+        fast = (os.environ.get("JANGQ_FORCE_SIMPLE_GEMV", "")[:1] != "1" and l0.bits != 5 and l0.group_size in (64, 128) and
+                l0.in_features // l0.group_size % 4 == 0 and
+                all(l.scales.dtype == self.dtype and l.weight.data_ptr() % 16 == 0 and l.scales.data_ptr() % 8 == 0 and
+                    l.biases.data_ptr() % 8 == 0 for l in run))
+        if not fast:
+            return len(run) * steps
+        forced = os.environ.get("JANGQ_GEMV_KERNEL", "")[:1] in ("m", "t", "p", "o")
+        return steps if forced else 1
 
     def _streamable(self, group) -> bool:
         lins = [self.linears[i] for i in group]

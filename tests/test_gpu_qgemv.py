@@ -456,3 +456,35 @@ def test_one_row_of_any_pitch(monkeypatch, form):
     want = jq.quantized_matmul(x, wq, s, b, group_size=64, bits=4)
     assert torch.equal(jq.quantized_matmul(view, wq, s, b, group_size=64, bits=4), want)
     assert pitches == [K, K]
+
+
+@pytest.mark.parametrize("m", (1, 8, 9, 16))
+@pytest.mark.parametrize("form", ("plain", "five_bit", "odd_groups", "other_sidecars", "unaligned", "forced", "simple", "nine"))
+def test_plan_counts_its_launches(monkeypatch, form, m):
+    """launches_per_run is the number of kernels in the plan's graph, on the fast kernels and off them."""
+    from cuda.bindings import runtime as rt
+    if form == "forced":
+        monkeypatch.setenv("JANGQ_GEMV_KERNEL", "mma")
+    if form == "simple":
+        monkeypatch.setenv("JANGQ_FORCE_SIMPLE_GEMV", "1")
+    K = 320 if form == "odd_groups" else 512
+    bits = {"five_bit": [5] * 5, "nine": [4] * 2 + [8] * 7}.get(form, [4, 4, 8, 4, 4])
+    lins = [jq.JANGLinear.from_float((torch.randn(96, K, device=DEV) * 0.02).bfloat16(), bits=b, group_size=64) for b in bits]
+    if form == "other_sidecars":
+        for l in lins:
+            l.scales, l.biases = l.scales.half(), l.biases.half()
+    if form == "unaligned":
+        flat = torch.empty(lins[1].scales.numel() + 1, dtype=torch.bfloat16, device=DEV)
+        flat[1:] = lins[1].scales.reshape(-1)
+        lins[1].scales = flat[1:].view_as(lins[1].scales)
+    plan = jq.GemvPlan(lins, m=m, device=DEV, groups=[list(range(len(lins)))])
+    plan._enqueue()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        plan._enqueue()
+    handle = rt.cudaGraph_t(init_value=graph.raw_cuda_graph())
+    _, _, count = rt.cudaGraphGetNodes(handle, 0)
+    _, nodes, _ = rt.cudaGraphGetNodes(handle, count)
+    kinds = [rt.cudaGraphNodeGetType(n)[1] for n in nodes]
+    assert kinds.count(rt.cudaGraphNodeType.cudaGraphNodeTypeKernel) == plan.launches_per_run == len(kinds)
