@@ -299,7 +299,7 @@ qgemm_ts_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
         int buf = 0, slot = 0;
         uint32_t phase = 1u;
         const SideSrc side = {a.scales, a.biases, nullptr, nullptr, a.G, side_mode(a.scales, a.biases, a.G, a.gs)};
-        ok = load_codes<BITS, 1, CD>(a.codes, n0, a.N, a.K, kb0 / CKB, nst, sC, cfull, cempty, threadIdx.x - 64, buf, phase, side,
+        ok = load_codes<BITS, CD>(a.codes, n0, a.N, a.K, kb0 / CKB, nst, sC, cfull, cempty, threadIdx.x - 64, buf, phase, side,
                                      sSide, slot);
         cp_async_commit();
         cp_async_wait<0>();
@@ -571,7 +571,7 @@ qgemm_pers_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs a) {
             const PersTile t = take(tile);
             if (t.rows <= 0) continue;
             const SideSrc side = {t.scales, t.biases, t.scales2, t.biases2, a.G, pers_side_mode<GU>(a, t)};
-            ok = load_codes<BITS, 1, CD, GU>(t.codes, t.n0, a.N, a.K, 0, nst, sC, cfull, cempty, threadIdx.x - 64, buf, ph, side,
+            ok = load_codes<BITS, CD, GU>(t.codes, t.n0, a.N, a.K, 0, nst, sC, cfull, cempty, threadIdx.x - 64, buf, ph, side,
                                              smem + C::SIDE_OFF, slot, t.codes2);
         }
         cp_async_commit();

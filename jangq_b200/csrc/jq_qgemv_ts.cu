@@ -140,7 +140,7 @@ qgemv_ts_kernel(const __grid_constant__ CUtensorMap xmap, const GemvArgs a, cons
         int buf = 0, slot = 0;
         uint32_t phase = 1u;
         const SideSrc side = {bt.scales[mi], bt.biases[mi], nullptr, nullptr, a.G, a.gs_shift ? 3 : 1};
-        ok = load_codes<BITS, 1, CD>(bt.codes[mi], n0, N, a.K, kb0 / CKB, nst, sC, cfull, cempty, threadIdx.x - 64, buf,
+        ok = load_codes<BITS, CD>(bt.codes[mi], n0, N, a.K, kb0 / CKB, nst, sC, cfull, cempty, threadIdx.x - 64, buf,
                                      phase, side, smem + C::SIDE_OFF, slot);
         cp_async_commit();
         cp_async_wait<0>();

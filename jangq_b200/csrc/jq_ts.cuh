@@ -308,7 +308,7 @@ template <int N> __device__ __forceinline__ void cp_async_small(uint32_t dst, co
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(N) : "memory");
 }
 
-// The loader warps' loop: 64 lanes (l) copy nst stages of 128*WT rows, starting at stage st0 of the rows, into a ring
+// The loader warps' loop: 64 lanes (l) copy nst stages of 128 rows, starting at stage st0 of the rows, into a ring
 // of CD stages; consecutive lanes take consecutive 16-byte chunks of a row, completion is counted on cfull (64
 // arrivals).  A lane's chunks keep their rows and columns from stage to stage, so only one multiply-add and one copy per
 // chunk are left in the loop (a warp alone on its scheduler issues an instruction every ~6 cycles;
@@ -316,15 +316,15 @@ template <int N> __device__ __forceinline__ void cp_async_small(uint32_t dst, co
 // (0, 1) at the start: the first pass finds every stage empty.  Returns false when a wait ran out; the caller waits for
 // the copies in flight.
 //   codes2 (PAIR): the tile is rows [n0, n0 + 64) of two matrices, the second one's behind the first one's
-template <int BITS, int WT, int CD, bool PAIR = false>
+template <int BITS, int CD, bool PAIR = false>
 __device__ __forceinline__ bool load_codes(const uint32_t* codes, int64_t n0, int64_t N, int64_t K, int st0, int nst,
                                            uint8_t* sC, uint64_t* cfull, uint64_t* cempty, int l, int& buf,
                                            uint32_t& phase, const SideSrc& side, uint8_t* sSide, int& slot,
                                            const uint32_t* codes2 = nullptr) {
     constexpr int RB = CodeStage<BITS>::RB, CPR = RB / 16;
-    constexpr int NCH = 128 * WT * CPR / 64;                               // chunks per lane and stage
+    constexpr int NCH = 128 * CPR / 64;                               // chunks per lane and stage
     const uint32_t rowbytes = (uint32_t)(K * BITS / 8);
-    const int last = (int)min((int64_t)((PAIR ? 64 : 128 * WT) - 1), N - 1 - n0);       // rows past N repeat the last one
+    const int last = (int)min((int64_t)((PAIR ? 64 : 128) - 1), N - 1 - n0);       // rows past N repeat the last one
     const uint8_t* src = reinterpret_cast<const uint8_t*>(codes) + n0 * (int64_t)rowbytes + (int64_t)st0 * RB;
     const int64_t second = PAIR ? reinterpret_cast<const uint8_t*>(codes2) - reinterpret_cast<const uint8_t*>(codes) : 0;
     uint32_t row[NCH];
@@ -352,7 +352,7 @@ __device__ __forceinline__ bool load_codes(const uint32_t* codes, int64_t n0, in
     for (int st = 0; st < nst; ++st) {
         ok = __all_sync(0xFFFFFFFFu, ts_wait(cempty + buf, phase));
         if (!ok) break;
-        const uint32_t d = dst0 + (uint32_t)(buf * (128 * WT * RB));
+        const uint32_t d = dst0 + (uint32_t)(buf * (128 * RB));
 #pragma unroll
         for (int j = 0; j < NCH; ++j) {
             const uint32_t dj = d + (uint32_t)(j * 1024);
