@@ -888,3 +888,76 @@ def test_grouped_gemm_of_256_row_tiles(bits, K):
     fused = [gate_up(x, sp, gate, up) for sp in lists]
     assert all(torch.equal(plain[0], p) for p in plain[1:]) and all(torch.equal(fused[0], f) for f in fused[1:])
     _lib.check(_lib.load().jq_device_status())
+
+
+def products(x, idx, ws):
+    """float64 x[p] . w[idx[p]]^T over weights rounded to x's type, expert by expert."""
+    y = torch.zeros((x.shape[0], ws[0].shape[0]), dtype=torch.float64, device=DEV)
+    for e, w in enumerate(ws):
+        rows = idx == e
+        if bool(rows.any()):
+            y[rows] = x[rows].double() @ w.double().T
+    return y
+
+
+@pytest.mark.parametrize("bits,K,gs,dtype", (
+    (2, 640, 64, torch.bfloat16),      # ten k-blocks: the groups rotate by two; stages of four, the last one half
+    (2, 1152, 128, torch.bfloat16),    # nine groups a row: sidecars not staged
+    (3, 640, 128, torch.float16),
+    (4, 1152, 64, torch.bfloat16),     # eighteen k-blocks: two 4-byte sidecar copies a chunk, the last one half
+    (4, 320, 64, torch.float16),       # five k-blocks: rotation by one, five groups a row
+    (5, 640, 64, torch.bfloat16),
+    (5, 384, 32, torch.float16),       # groups of 32: two scales a k-block, the general expansion
+    (6, 320, 64, torch.float16),
+    (8, 192, 32, torch.bfloat16),      # three k-blocks: rotation by three
+    (8, 1024, 128, torch.bfloat16),
+))
+def test_grouped_gemm_walk_over_many_tiles(bits, K, gs, dtype):
+    """Several tiles per CTA (64 experts x 9 column tiles on 148 SMs, twice that with gate and up), so that the state carried
+    from tile to tile -- k-block rotation, code and sidecar ring positions, accumulators -- takes all its values: against
+    float64 over the same rounded weights.  Bound: one rounding of the output and 1e-3 of the largest value (float32
+    sums, and a weight whose float32 value ties between two 16-bit ones)."""
+    E, N = 64, 1104
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(bits * K + gs)
+    banks, ws = [], []
+    for _ in range(2):
+        packed = jq.quantize((torch.randn((E, N, K), generator=gen, device=DEV) * 0.1).to(dtype), gs, bits)
+        banks.append(jq.ExpertBank(*packed, bits, gs))
+        ws.append(jq.dequantize(*packed, gs, bits, dtype=torch.float32).to(dtype))
+    counts = torch.randint(0, 70, (E,), generator=gen, device=DEV)
+    counts[5], counts[40] = 300, 193
+    idx = torch.repeat_interleave(torch.arange(E, device=DEV, dtype=torch.int32), counts)
+    x = torch.randn((idx.numel(), K), generator=gen, device=DEV).to(dtype)
+    g, u = products(x, idx, ws[0]), products(x, idx, ws[1])
+    h = g / (1 + torch.exp(-g)) * u
+    ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    for tile_m in (128, 192, 256) if dtype == torch.bfloat16 else (128, 192):
+        sp = SortedPairs(idx, E, tile_m=tile_m)
+        for got, ref in ((grouped(x, sp, banks[0]), g), (gate_up(x, sp, *banks), h)):
+            assert torch.all((got.double() - ref).abs() <= ulp * ref.abs() + 1e-3 * ref.abs().max())
+    _lib.check(_lib.load().jq_device_status())
+
+
+@pytest.mark.parametrize("tile_m", (128, 192, 256))
+def test_grouped_gemm_walk_over_mixed_widths(tile_m):
+    """Experts of five widths in one list: each launch walks all tiles and takes those of its width, the skipped ones lie
+    between them."""
+    E, N, K, gs = 60, 1152, 640, 64
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(tile_m)
+    experts, ws = [], []
+    for e in range(E):
+        b = (2, 3, 8, 4, 6)[e * 7 // 4 % 5]
+        packed = jq.quantize((torch.randn((N, K), generator=gen, device=DEV) * 0.1).bfloat16(), gs, b)
+        experts.append((*packed, b))
+        ws.append(jq.dequantize(*packed, gs, b, dtype=torch.float32).bfloat16())
+    bank = jq.ExpertBank.from_experts(experts, gs)
+    counts = torch.randint(0, 70, (E,), generator=gen, device=DEV)
+    counts[7] = 500
+    idx = torch.repeat_interleave(torch.arange(E, device=DEV, dtype=torch.int32), counts)
+    x = torch.randn((idx.numel(), K), generator=gen, device=DEV).bfloat16()
+    ref = products(x, idx, ws)
+    got = grouped(x, SortedPairs(idx, E, tile_m=tile_m), bank).double()
+    assert torch.all((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-3 * ref.abs().max())
+    _lib.check(_lib.load().jq_device_status())

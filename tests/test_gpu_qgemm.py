@@ -114,9 +114,9 @@ def test_device_status_clean_after_gemm():
 
 @pytest.mark.parametrize("gs", (64, 128))
 @pytest.mark.parametrize("bits", (2, 3, 4, 5, 6, 8))
-def test_qgemm_two_row_tiles_per_cta(bits, gs):
-    """Shapes large enough for the two-accumulator form (256 rows of the activations per CTA): a ragged last
-    row tile whose second half is empty, a ragged last column tile, every width and code-stage layout."""
+def test_qgemm_several_row_tiles(bits, gs):
+    """Five row tiles and 58 column tiles (two waves): a ragged last tile in both directions, every width and code-stage
+    layout."""
     M, N, K = 1160, 7300, 384
     x, wq, s, b = make_case(M, N, K, bits, gs, torch.bfloat16, seed=bits + gs)
     y = jq.quantized_matmul(x, wq, s, b, group_size=gs, bits=bits)
@@ -124,15 +124,18 @@ def test_qgemm_two_row_tiles_per_cta(bits, gs):
     _lib.check(_lib.load().jq_device_status())
 
 
-def test_qgemm_two_row_tiles_equal_one_row_tile_results():
-    """The same rows through the one- and the two-accumulator form (a small N keeps one tile per CTA) are
-    bit-identical: the accumulation order along K is the same."""
-    M, K, bits, gs = 1024, 512, 4, 64
-    x, wq, s, b = make_case(M, 8192, K, bits, gs, torch.bfloat16, seed=5)
-    y2 = jq.quantized_matmul(x, wq, s, b, group_size=gs, bits=bits)                  # 32 x 4 CTAs: two tiles each
-    y1 = jq.quantized_matmul(x, wq[:512].contiguous(), s[:512].contiguous(), b[:512].contiguous(), group_size=gs,
-                             bits=bits)                                               # 2 x 8 CTAs: one tile each
-    assert torch.equal(y2[:, :512], y1)
+@pytest.mark.parametrize("bits,K", ((2, 512), (3, 384), (8, 320)))
+def test_grouped_and_dense_gemm_agree_bit_for_bit(bits, K):
+    """The persistent grouped kernel (one expert, tiles of 128, 192 and 256 rows) and the one-tile dense kernel, unsplit for
+    fewer than sixteen k-blocks, sum the same operands in the same order."""
+    from jangq_b200.moe import ExpertBank, SortedPairs, _moe_gemm
+    M, N, gs = 1000, 8192, 64
+    x, wq, s, b = make_case(M, N, K, bits, gs, torch.bfloat16, seed=5)
+    y = jq.quantized_matmul(x, wq, s, b, group_size=gs, bits=bits)
+    bank = ExpertBank(wq[None], s[None], b[None], bits, gs)
+    idx = torch.zeros((M,), dtype=torch.int32, device=DEV)
+    for tile_m in (128, 192, 256):
+        assert torch.equal(_moe_gemm(x, SortedPairs(idx, 1, tile_m=tile_m), bank), y)
 
 
 @pytest.mark.parametrize("bits", (2, 3, 4, 5, 6, 8))
@@ -172,27 +175,46 @@ def test_qgemm_expansion_and_sidecar_forms(M, N, K, gs, scale, bits, dtype):
     _lib.check(_lib.load().jq_device_status())
 
 
+def round_to(v, dtype):
+    """float64 -> the 16-bit type's nearest value (ties to even, subnormals), as float64.  torch goes through float32."""
+    p, emin = (8, -125) if dtype == torch.bfloat16 else (11, -13)
+    quantum = np.ldexp(1.0, np.maximum(np.frexp(v)[1], emin) - p)
+    return np.rint(v / quantum) * quantum
+
+
 @pytest.mark.parametrize("dtype", (torch.bfloat16, torch.float16))
+@pytest.mark.parametrize("gs", (32, 64, 128))
 @pytest.mark.parametrize("bits", (2, 3, 4, 5, 6, 8))
-def test_qgemm_weight_operand_is_rounded_once(bits, dtype):
-    """x = identity returns the weight operand itself: rn(q * scale + bias), the dequantizer's values, bit for bit --
-    over scales from the subnormals of the activation type to above the limit of the fast expansion.  (8-bit codes of
-    large bfloat16 scales go through float32 and may round twice: one step.)"""
-    K, N, gs = 256, 192, 64
-    rng = np.random.default_rng(bits)
-    mag = np.exp2(rng.uniform(-12 if dtype == torch.float16 else -100, 6, size=(N, K // gs, 1)))
-    w = torch.from_numpy((rng.standard_normal((N, K // gs, gs)) * mag).astype(np.float32).reshape(N, K)).to(DEV).to(dtype)
-    wq, s, b = jq.quantize(w, gs, bits)
-    y = jq.quantized_matmul(torch.eye(K, dtype=dtype, device=DEV), wq, s, b, group_size=gs, bits=bits)
-    ref = jq.dequantize(wq, s, b, gs, bits, dtype=torch.float32).to(dtype).T
-    # -0 and +0 meet in the sum; a product with a subnormal weight is exact in the float32 accumulator
-    if bits == 8 and dtype == torch.bfloat16:
-        assert torch.all((y.float() - ref.float()).abs() <= ref.float().abs() * 2.0 ** -7 + 1e-38)
+def test_qgemm_weight_operand_is_rounded_once(bits, gs, dtype):
+    """x = identity returns the weight operand itself: rn(q * scale + bias), one rounding, bit for bit.  The expansion is
+    chosen per 32 rows and k-block (the rows of a warp), so the magnitude of the scales is drawn for such blocks: all at the
+    bottom of the type (float16: subnormal; bfloat16: far below one), all small, all just below the limit of the fast form, all above it, and rows on
+    both sides.  The one exception, 8-bit codes with bfloat16 in the general form (groups of 32, or a scale of the warp at
+    2^-5 or above), rounds to float32 first."""
+    bf = dtype == torch.bfloat16
+    K, N = 512, 320                                       # ten blocks of 32 rows, the last tile half full
+    rng = np.random.default_rng(bits + gs)
+    if bf:
+        limit = {2: -1, 3: 0, 4: -5, 5: -2, 6: -3, 8: -5}[bits]
+        classes = ((-100, -90), (-40, -8), (limit - 3, limit), (limit, limit + 8), (limit - 2, limit + 2))
     else:
-        exact = jq.dequantize(wq, s, b, gs, bits, dtype=torch.float32).T.double()
-        # the dequantizer rounds to float32 and then to 16 bits, the operand once: either neighbour of a tie
-        ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
-        assert torch.all((y.double() - exact).abs() <= exact.abs() * ulp * (1 + 1e-4) + 6.1e-8 * (dtype == torch.float16))
+        limit = {2: -2, 3: 0, 4: -4, 5: -2, 6: -3, 8: 4}[bits]       # 8-bit: no limit
+        classes = ((-24, -14), (-14, -8), (limit - 3, limit - 0.05), (limit, limit + 3), (limit - 2, limit + 2))
+    kb = max(gs, 64)
+    which = rng.integers(0, len(classes), (N // 32, K // kb)).repeat(32, 0).repeat(kb // gs, 1)
+    lo, hi = np.array(classes)[which].transpose(2, 0, 1)
+    s = torch.from_numpy(np.exp2(rng.uniform(lo, hi)) * rng.choice([-1.0, 1.0], lo.shape)).to(DEV).to(dtype)
+    sv = s.double().cpu().numpy()
+    b = torch.from_numpy(sv * rng.uniform(-2.0 ** bits, 2.0, sv.shape)).to(DEV).to(dtype)
+    q = rng.integers(0, 2 ** bits, (N, K))
+    wq = torch.from_numpy(jo.pack_rows(q, bits).view(np.int32)).to(DEV)
+    exact = q * sv.repeat(gs, 1) + b.double().cpu().numpy().repeat(gs, 1)        # 53 bits hold it
+    if bf and bits == 8:
+        general = np.abs(sv).reshape(N // 32, 32, K // kb, -1).max((1, 3)) >= 2.0 ** -5 if gs >= 64 else np.ones((N // 32, K // kb), bool)
+        exact = np.where(general.repeat(32, 0).repeat(kb, 1), exact.astype(np.float32).astype(np.float64), exact)
+    y = jq.quantized_matmul(torch.eye(K, dtype=dtype, device=DEV), wq, s, b, group_size=gs, bits=bits)
+    assert np.array_equal(y.double().cpu().numpy().T, round_to(exact, dtype))
+    _lib.check(_lib.load().jq_device_status())
 
 
 @pytest.mark.parametrize("M", (16, 17))
