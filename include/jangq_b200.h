@@ -201,8 +201,9 @@ int jq_qgemv_stream_run(const JqStreamProgram* program, jq_stream_t stream);
  * activation rows (MLX switches from qmv to its tiled qmm there; the reference's only
  * statement of that kernel is the tile shape at jang_tools/jangh/kernels.py:34,273-277).
  * Y[M,N] = X[M,K] . deq(W)[N,K]^T on tcgen05 tensor cores: the weights are dequantized to
- * the activation type (one rounding) tile by tile in shared memory, f32 accumulation in
- * tensor memory.  Needs K % 64 == 0 and x/scales/biases/y of the same 16-bit type. */
+ * the activation type in registers and are the A operand in tensor memory, f32 accumulation there.
+ * One rounding per weight; two (float32 first) for 8-bit codes with bf16 where a scale of 32
+ * neighbouring rows and 64 columns is 2^-5 or more, or group_size is 32.  Needs K % 64 == 0 and x/scales/biases/y of the same 16-bit type. */
 int jq_qgemm(const void* x, int x_dtype, int64_t M, int64_t ldx, const uint32_t* codes,
              const void* scales, const void* biases, int sidecar_dtype, int64_t N, int64_t K,
              int bits, int group_size, void* y, int y_dtype, int64_t ldy, jq_stream_t stream);

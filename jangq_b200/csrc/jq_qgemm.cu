@@ -26,7 +26,8 @@
 // tile as the B operand in shared memory, one thread per weight row, one group of dequantizer warps).
 //
 // Numerics: the A operand is the dequantized weight rounded once to the activation type (what
-// MLX's qmm feeds its matrix units), products are accumulated in f32 in ascending k order.
+// MLX's qmm feeds its matrix units), products are accumulated in f32 in ascending k order.  8-bit codes with bf16 round
+// to f32 first in the general form of the expansion (groups of 32, or a scale of the warp's rows at 2^-5 or above).
 #include <cuda.h>
 
 #include <algorithm>
@@ -54,8 +55,8 @@ struct GemmArgs {
     int y_pair_ok;   // rows of y are 4-byte aligned
     int y_vec_ok;    // rows of y are 8-byte aligned
     int* status;     // device status word, set to 1 when a bounded wait ran out
-    // grouped mode (routed experts): blockIdx.y indexes a tile list built by jq_moe_sort; rows are the
-    // expert-sorted (token, slot) pairs, weights come from per-expert pointer tables
+    // grouped mode (routed experts): CTAs walk a tile list built by jq_moe_sort; rows are the expert-sorted
+    // (token, slot) pairs, weights come from per-expert pointer tables
     const int32_t* tile_expert;
     const int32_t* tile_row0;
     const int32_t* num_tiles;
