@@ -356,10 +356,11 @@ int resident_clusters(int S, int per_sm) {
 }
 
 // Cluster size along K with the shortest estimated time (us): of two CTAs on an SM each walks a k-block in 0.52 us and
-// a round of them starts and ends in 3.6 us, one alone takes 0.33 and 4.4, and a split adds the exchange of the sums, more
-// with every round.  Measured on B200 over 4 to 460 row blocks, 2- to 8-bit codes, 6 to 16 rows (all scale alike).  The
-// largest split that one round holds, as before, left half of the chip idle between one and 1.4 row blocks per SM (9 rows,
-// 22016x4096 2-bit, group 128: 40.5 us unsplit, 36.5 by 3; 16 rows, 9600x11264 6-bit: 66.5 by 2, 48.7 by 3).
+// a round of them starts and ends in 3.6 us (4.2 where four or more split K), one alone takes 0.33 (and 4.4), and a split
+// adds the exchange of the sums, more with every round.  Measured on B200 over 4 to 460 row blocks, 2- to 8-bit codes, 6
+// to 16 rows (all scale alike).  The largest split that one round holds, as before, left half of the chip idle between
+// one and 1.4 row blocks per SM (9 rows, 22016x4096 2-bit, group 128: 40.5 us unsplit, 36.5 by 3; 16 rows, 9600x11264
+// 6-bit: 66.5 by 2, 48.7 by 3).
 TsSplit ts_split(int64_t row_blocks, int64_t K) {
     TsSplit best = {1, 1e30f};
     const int64_t chunks = K / 256;                        // of four k-blocks: what a split deals out
@@ -369,8 +370,8 @@ TsSplit ts_split(int64_t row_blocks, int64_t K) {
         const float pairs = (float)(row_blocks / two + (rest > one ? 1 : 0)), single = rest > 0 && rest <= one ? 1.f : 0.f;
         const float k = (float)((chunks + S - 1) / S) * 4.f;
         const float exchange = S == 1 ? 0.f : S == 2 ? 1.0f : S == 3 ? 2.5f : S == 4 ? 1.3f : 2.0f;
-        const float us = pairs * (0.52f * k + 3.6f) + single * (0.33f * k + 4.4f) + exchange * (0.4f + 0.6f * (pairs + single)) +
-                         (S >= 4 ? 0.6f * pairs : 0.f);
+        const float us = pairs * (0.52f * k + (S < 4 ? 3.6f : 4.2f)) + single * (0.33f * k + (S < 4 ? 3.6f : 4.4f)) +
+                         exchange * (0.4f + 0.6f * (pairs + single));
         if (us < best.us) best = {S, us};
     }
     return best;
