@@ -218,7 +218,8 @@ def _qgemv(x2: torch.Tensor, wq, scales, biases, K, bits, group_size, out: torch
     lib = _lib.load()
     dev = x2.device
     M, N = x2.shape[0], wq.shape[0]
-    _lib.check(lib.jq_qgemv_ex(x2.data_ptr(), _lib.dtype_id(x2.dtype), M, x2.stride(0), wq.data_ptr(),
+    # the pitch of a single row is whatever the view it came from had (a transposed column has 1) and says nothing
+    _lib.check(lib.jq_qgemv_ex(x2.data_ptr(), _lib.dtype_id(x2.dtype), M, x2.stride(0) if M > 1 else K, wq.data_ptr(),
                                scales.data_ptr(), biases.data_ptr(), _lib.dtype_id(scales.dtype), N, K, bits,
                                group_size, out.data_ptr(), _lib.dtype_id(out.dtype), out.stride(0), flags,
                                _lib.stream_ptr(dev)))
@@ -297,8 +298,7 @@ def quantized_matmul(x: torch.Tensor, w: torch.Tensor, scales: torch.Tensor, bia
     if x.dtype not in (torch.bfloat16, torch.float16):
         raise JangqError(_lib.JQ_EINVAL, f"activations must be bfloat16 or float16, got {x.dtype}")
     matrix = len(xshape) == 2
-    # the pitch of a single row is whatever the view it came from had (a transposed column has 1): a reshape sets it to K
-    x2 = x if matrix and (xshape[0] != 1 or x.stride(0) == K) else x.reshape(-1, K)
+    x2 = x if matrix else x.reshape(-1, K)
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
     M, N = x2.shape[0], w.shape[0]

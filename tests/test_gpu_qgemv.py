@@ -444,15 +444,23 @@ def test_small_batch_kernel(M, N, K, gs, bits, dtype):
 def test_one_row_of_any_pitch(monkeypatch, form):
     """The stride between rows of a one-row input says nothing: a transposed column (1), an expanded vector and a row of
     a buffer with an odd pitch are taken as a row of K, by the kernel that a contiguous row gets."""
-    from jangq_b200 import ops
     K = 256
     x, wq, s, b = make_case(96, K, 4, 64, 1, torch.bfloat16, seed=7)
     view = {"column": x.reshape(K, 1).t(), "expanded": torch.as_strided(x, (1, K), (0, 1)),
             "padded": torch.nn.functional.pad(x, (0, 3))[:, :K]}[form]
     assert view.shape == (1, K) and view.stride(0) != K
     pitches = []
-    qgemv = ops._qgemv
-    monkeypatch.setattr(ops, "_qgemv", lambda x2, *a: (pitches.append(x2.stride(0)), qgemv(x2, *a)))
+    lib = _lib.load()
+
+    class Recorder:
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def jq_qgemv_ex(self, *a):
+            pitches.append(a[3])
+            return lib.jq_qgemv_ex(*a)
+
+    monkeypatch.setattr(_lib, "load", Recorder)
     want = jq.quantized_matmul(x, wq, s, b, group_size=64, bits=4)
     assert torch.equal(jq.quantized_matmul(view, wq, s, b, group_size=64, bits=4), want)
     assert pitches == [K, K]
