@@ -155,12 +155,14 @@ def dtype_id(dt: torch.dtype) -> int:
 # torch.device objects in the checks.  Both functions are private to torch; its public ones serve where it lacks them.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_ordinal = {torch.device("cuda", i): i for i in range(64)}     # one look-up instead of type and index of a device
 
 
 def stream_ptr(device=None) -> int:
     """Handle of the current stream of `device` (a torch.device, an ordinal, a string; None: the current device)."""
-    if _raw_stream is not None and isinstance(device, torch.device) and device.type == "cuda" and device.index is not None:
-        return _raw_stream(device.index)
+    index = _ordinal.get(device)
+    if index is not None and _raw_stream is not None:
+        return _raw_stream(index)
     return torch.cuda.current_stream(device).cuda_stream
 
 
