@@ -600,7 +600,8 @@ float tc_estimate_us(int64_t row_blocks, int64_t K, int gs, int64_t M, int act_d
     if (slice > 4096 || row_blocks > resident_clusters(S, 1)) return 1e30f;
     const float r = (float)(M - 6);
     const float per64 = gs == 128 ? 0.25f + 0.015f * r : act_dtype == JQ_F16 ? 0.285f + 0.0165f * r : 0.3275f + 0.0125f * r;
-    const float sum = S == 1 ? 0.f : (S == 2 ? 1.6f : S < 5 ? (float)S - 0.5f : 5.5f) + (gs == 64 ? 1.5f : 0.f);
+    float sum = S == 1 ? 0.f : (S == 2 ? 1.6f : S < 5 ? 3.6f : 5.5f) + (gs == 64 ? 1.5f : 0.f);
+    if (S > 1 && slice > 3072) sum += 1.5f;
     const float k = (float)(slice / 64), walk = k * per64 + 2.6f, least = S < 3 ? k * 0.19f + 4.6f : 0.f;
     return (walk > least ? walk : least) + sum;
 }
